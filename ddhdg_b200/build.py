@@ -3,17 +3,19 @@
 import os
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libddhdg_b200.so")
-SOURCES = ["hdg_capi.cu"]
+# compiled side by side, one object per source
+SOURCES = ["hdg_capi.cu", "hdg_ndsolve.cu"]
 HEADER = os.path.join(HERE, "..", "include", "ddhdg_b200.h")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC",
 ]
 
 
@@ -33,11 +35,21 @@ def needs_build():
 def build(force=False, verbose=False):
     if not force and not needs_build():
         return LIB
-    cmd = [nvcc()] + NVCC_FLAGS + ["-o", LIB] + [os.path.join(CSRC, s) for s in SOURCES] + \
-        ["-lcusolver", "-lcusparse", "-lcublas"]
-    if verbose:
-        print(" ".join(cmd), file=sys.stderr)
-    subprocess.check_call(cmd)
+    with tempfile.TemporaryDirectory() as tmp:
+        objs, jobs = [], []
+        for s in SOURCES:
+            objs.append(os.path.join(tmp, s + ".o"))
+            cmd = [nvcc()] + NVCC_FLAGS + ["-c", "-o", objs[-1], os.path.join(CSRC, s)]
+            if verbose:
+                print(" ".join(cmd), file=sys.stderr)
+            jobs.append((cmd, subprocess.Popen(cmd)))
+        for cmd, job in jobs:
+            if job.wait():
+                raise subprocess.CalledProcessError(job.returncode, cmd)
+        cmd = [nvcc()] + NVCC_FLAGS + ["-shared", "-o", LIB] + objs + ["-lcusolver", "-lcusparse"]
+        if verbose:
+            print(" ".join(cmd), file=sys.stderr)
+        subprocess.check_call(cmd)
     return LIB
 
 

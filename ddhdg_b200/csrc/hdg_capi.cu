@@ -25,7 +25,7 @@
 #include "hdg_condense.cuh"
 #include "hdg_condense3.cuh"
 #include "hdg_kernels.cuh"
-#include "hdg_ndsolve.cuh"
+#include "hdg_ndsolve.h"
 #include "hdg_plain.cuh"
 #include "hdg_tables.h"
 

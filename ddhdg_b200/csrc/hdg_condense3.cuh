@@ -21,20 +21,11 @@
 #include <cuda_runtime.h>
 
 #include "hdg_condense.cuh"
+#include "hdg_mma.cuh"
 
 namespace ddhdg
 {
   constexpr int Condense3MaxWPB = 8; // warps (cells) per CTA at most
-
-  // D += A B for one 8x8x4 FP64 tile on the tensor path (mma.sync m8n8k4):
-  // lane l holds A[l/4][l%4], B[l%4][l/4] and D[l/4][2(l%4) + {0,1}]
-  __device__ __forceinline__ void
-  dmma8x8x4(double &d0, double &d1, double a, double b)
-  {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-  }
 
   // row stride of the staged S^-1 (>= its padded width, = 4 mod 16 doubles:
   // the A-fragment loads of a half warp hit 16 different 8-byte banks)

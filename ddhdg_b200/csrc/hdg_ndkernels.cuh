@@ -1,0 +1,1374 @@
+// Device kernels of the nested-dissection trace solve (sm_100a, FP64); the
+// tree, the batches and the launch sequence are in hdg_ndsolve.cu.
+//
+// A tree node eliminates its nE dofs (E) against its nK kept dofs (K).  What
+// stays of a front in memory is its K columns and the right-hand-side
+// column, [E rows | K rows] x (nK + 1), column-major with leading dimension
+// ld: W = F_EE^-1 [F_EK | r_E] in the E rows and the Schur complement
+// F_KK - F_KE W in the K rows.  The E columns live in scratch while the
+// node's batch is eliminated.  Every front entry is the sum of at most two
+// entries of the children's Schur complements, read through the maps of the
+// node's shape where it is needed (no zeroed front, no extend-add pass):
+// an E face touches both children, a K face exactly one.  Children that are
+// interior cells are read directly from the condensed blocks.
+#pragma once
+
+#include <cooperative_groups.h>
+#include <cstdint>
+#include <cuda_runtime.h>
+
+#include "hdg_mma.cuh"
+
+namespace ddhdg
+{
+  struct NDNode
+  {
+    int64_t koff;     // K columns of the front (doubles)
+    int64_t eoff;     // E columns in the batch's scratch
+    int64_t luoff;    // LU factors in the batch's scratch
+    int64_t tioff;    // inverted diagonal blocks in the batch's scratch
+    int64_t coff[2];  // the children's K columns
+    int64_t ccell[2]; // cell of a child read from the condensed blocks, or -1
+    int64_t cell;     // the node's cell (leaf), or -1
+    int64_t doff;     // dof list [E, K]
+    int64_t poff;     // pivot order and row lists in the batch's scratch
+    int32_t map;      // maps of the node's shape
+    int32_t nE, nK;
+    int32_t nEp; // nE rounded up to even: first K row
+    int32_t ld;  // nEp + nK rounded up to even
+    int32_t cEp[2], cld[2], cnK[2];
+  };
+
+  // the condensed per-cell blocks and the row scaling
+  struct NDCells
+  {
+    const double  *tt, *rhs, *dval, *dscale;
+    const int32_t *dflag;
+    const int64_t *cell_faces;
+    int            Nt, nd, F;
+  };
+
+  constexpr int NDKidBit = 30; // maps of the K rows: child << 30 | kept index
+
+  // rows of the trace matrix: max |tt[a][:]| per global dof (bit pattern of a
+  // non-negative double, so that an integer max is the double max)
+  __global__ void
+  nd_rowmax_kernel(int64_t ncells, NDCells C, unsigned long long *dmax)
+  {
+    const int64_t tot = ncells * C.Nt;
+    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < tot;
+         idx += (int64_t)gridDim.x * blockDim.x)
+      {
+        const int64_t cell = idx / C.Nt;
+        const int     a    = (int)(idx % C.Nt);
+        const double *row  = C.tt + (cell * C.Nt + a) * (int64_t)C.Nt;
+        double        m    = 0.;
+        for (int b = 0; b < C.Nt; ++b)
+          m = fmax(m, fabs(row[b]));
+        const int64_t g = C.cell_faces[cell * C.F + a / C.nd] * C.nd + a % C.nd;
+        atomicMax(dmax + g, (unsigned long long)__double_as_longlong(m));
+      }
+  }
+
+  __global__ void
+  nd_rowscale_kernel(int64_t n, const unsigned long long *dmax, double *dscale)
+  {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+      {
+        const double m = __longlong_as_double((long long)dmax[i]);
+        dscale[i]      = (m > 0.) ? 1. / m : 1.;
+      }
+  }
+
+  __device__ __forceinline__ double
+  nd_cell_scale(const NDCells &C, int64_t cell, int a)
+  {
+    return C.dscale[C.cell_faces[cell * C.F + a / C.nd] * C.nd + a % C.nd];
+  }
+
+  // entry (row a, column b) of a cell's block: scaled, Dirichlet rows identity
+  __device__ __forceinline__ double
+  nd_cell_entry(const NDCells &C, int64_t cell, int a, int b)
+  {
+    if (C.dflag[cell * C.Nt + a])
+      return a == b ? 1. : 0.;
+    return C.tt[(cell * C.Nt + a) * (int64_t)C.Nt + b] * nd_cell_scale(C, cell, a);
+  }
+
+  __device__ __forceinline__ double
+  nd_cell_rhs(const NDCells &C, int64_t cell, int a)
+  {
+    const int64_t i = cell * C.Nt + a;
+    return C.dflag[i] ? C.dval[i] : C.rhs[i] * nd_cell_scale(C, cell, a);
+  }
+
+  // entry (kept row jr, kept column jc) of child s
+  __device__ __forceinline__ double
+  nd_kid(const NDNode &n, const double *fronts, int s, int jr, int jc)
+  {
+    // selects, not indices: the node stays out of local memory
+    return fronts[(s ? n.coff[1] : n.coff[0]) + (int64_t)jc * (s ? n.cld[1] : n.cld[0]) +
+                  (s ? n.cEp[1] : n.cEp[0]) + jr];
+  }
+
+  // Front entries by position: rows and columns 0..nE-1 are E, column nK of
+  // the K columns is the right-hand side.  Used by the kernels of the larger
+  // fronts, whose children always keep their own fronts in memory.
+  struct NDFront
+  {
+    const NDNode  &n;
+    const NDCells &C;
+    const int32_t *map;
+    const double  *fronts;
+    __device__ __forceinline__ double
+    EE(int i, int j) const
+    {
+      if (n.cell >= 0)
+        return nd_cell_entry(C, n.cell, map[i], map[j]);
+      return nd_kid(n, fronts, 0, map[i], map[j]) + nd_kid(n, fronts, 1, map[n.nE + i], map[n.nE + j]);
+    }
+    __device__ __forceinline__ double
+    KE(int r, int j) const
+    {
+      if (n.cell >= 0)
+        return nd_cell_entry(C, n.cell, map[n.nE + r], map[j]);
+      const int k = map[2 * n.nE + r], s = k >> NDKidBit;
+      return nd_kid(n, fronts, s, k & ((1 << NDKidBit) - 1), map[s * n.nE + j]);
+    }
+    __device__ __forceinline__ double
+    EK(int i, int c) const // c == nK: the right-hand side
+    {
+      if (n.cell >= 0)
+        return c == n.nK ? nd_cell_rhs(C, n.cell, map[i]) : nd_cell_entry(C, n.cell, map[i], map[n.nE + c]);
+      if (c == n.nK)
+        return nd_kid(n, fronts, 0, map[i], n.cnK[0]) + nd_kid(n, fronts, 1, map[n.nE + i], n.cnK[1]);
+      const int k = map[2 * n.nE + c], s = k >> NDKidBit;
+      return nd_kid(n, fronts, s, map[s * n.nE + i], k & ((1 << NDKidBit) - 1));
+    }
+    __device__ __forceinline__ double
+    KK(int r, int c) const
+    {
+      if (n.cell >= 0)
+        return c == n.nK ? nd_cell_rhs(C, n.cell, map[n.nE + r]) :
+                           nd_cell_entry(C, n.cell, map[n.nE + r], map[n.nE + c]);
+      const int kr = map[2 * n.nE + r], sr = kr >> NDKidBit, jr = kr & ((1 << NDKidBit) - 1);
+      if (c == n.nK)
+        return nd_kid(n, fronts, sr, jr, sr ? n.cnK[1] : n.cnK[0]);
+      const int kc = map[2 * n.nE + c];
+      return (kc >> NDKidBit) == sr ? nd_kid(n, fronts, sr, jr, kc & ((1 << NDKidBit) - 1)) : 0.;
+    }
+  };
+
+  // 32-bit pivot key of a candidate: the high word of |x| (sign, exponent,
+  // 20 mantissa bits) plus one, so that 0 marks rows that cannot be chosen;
+  // the pivot is within 2^-20 of the largest candidate, ties go to the first
+  __device__ __forceinline__ unsigned
+  nd_pivot_key(double x)
+  {
+    return (unsigned)((unsigned long long)__double_as_longlong(fabs(x)) >> 32) + 1u;
+  }
+
+  // ------------------------------------------------------------ small fronts
+  // nE <= NEM <= 36: the whole elimination of a front in one CTA.
+  // - F_EE goes into the registers of warp 0 (one row per lane, two for
+  //   NEM > 32; unit rows beyond nE): LU with virtual partial pivoting, the
+  //   pivot search one warp max-reduction, the pivot row broadcast by
+  //   shuffles, no barrier; the other warps stage [F_EK | r_E] and -F_KE.
+  // - W: a thread per column, its nE entries in registers, the factors
+  //   broadcast from shared memory; no barrier between its steps.
+  // - F_KK - F_KE W: 16 x 32 warp tiles on the FP64 tensor path with the
+  //   children's entries as the initial accumulators, stored once.
+  // Bound by memory (the children's Schur complements in, W and the own one
+  // out) and, per front, by the nE dependent pivot steps; several CTAs per
+  // SM overlap the two.
+  __host__ __device__ constexpr int
+  nd_small_class(int nE)
+  {
+    return nE <= 4 ? 4 : nE <= 12 ? 12 : nE <= 20 ? 20 : nE <= 28 ? 28 : 36;
+  }
+
+  constexpr int NDSmallE = 36;
+
+  __host__ __device__ inline size_t
+  nd_small_smem(int NEM, int nK, int Nt)
+  {
+    // rows of Bs / Ks hold NEM doubles: NEM = 4 or 12 (mod 16), so the
+    // tensor-path fragments read distinct banks
+    return ((size_t)NEM * NEM + NEM + (size_t)(2 * nK + 1) * NEM + 2 * (size_t)Nt) * sizeof(double) +
+           ((size_t)nK + 3 * NEM) * sizeof(int);
+  }
+
+  template <int NEM, bool LEAF>
+  __global__ void __launch_bounds__(256)
+  nd_small_kernel(const NDNode *nodes, const int32_t *maps, NDCells C, int nKmax, int *sing, double *fronts)
+  {
+    extern __shared__ __align__(16) double sm[];
+    constexpr int LDW = NEM;
+    constexpr int RPL = NEM > 32 ? 2 : 1;
+    const NDNode  n   = nodes[blockIdx.x];
+    const int     nE = n.nE, nK = n.nK;
+    double       *LU   = sm;                       // factors, [column][pivot order]
+    double       *dinv = LU + NEM * NEM;           // 1 / U_jj
+    double       *Bs   = dinv + NEM;               // [column of K, r][E row]
+    double       *Ks   = Bs + (nKmax + 1) * LDW;   // -F_KE: [K row][E column]
+    double       *scs  = Ks + nKmax * LDW;         // row scales of cells read directly
+    int          *km   = reinterpret_cast<int *>(scs + 2 * C.Nt);
+    int          *e0   = km + nKmax;
+    int          *e1   = e0 + NEM;
+    int          *perm = e1 + NEM;
+    const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
+    const int32_t *map = maps + n.map;
+    if (LEAF)
+      {
+        for (int i = tid; i < nE; i += T)
+          e0[i] = map[i];
+        for (int i = tid; i < nK; i += T)
+          km[i] = map[nE + i];
+        for (int a = tid; a < C.Nt; a += T)
+          scs[a] = nd_cell_scale(C, n.cell, a);
+      }
+    else
+      {
+        for (int i = tid; i < nE; i += T)
+          {
+            e0[i] = map[i];
+            e1[i] = map[nE + i];
+          }
+        for (int i = tid; i < nK; i += T)
+          km[i] = map[2 * nE + i];
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+          if (n.ccell[s] >= 0)
+            for (int a = tid; a < C.Nt; a += T)
+              scs[s * C.Nt + a] = nd_cell_scale(C, n.ccell[s], a);
+      }
+    __syncthreads();
+    // entries by local indices of child s (or of the node's own cell);
+    // column -1 is the right-hand side
+    const auto kid = [&](int s, int jr, int jc) -> double {
+      const int64_t cell = s ? n.ccell[1] : n.ccell[0];
+      if (cell >= 0)
+        return (jc < 0 ? C.rhs[cell * C.Nt + jr] : C.tt[(cell * C.Nt + jr) * (int64_t)C.Nt + jc]) *
+               scs[s * C.Nt + jr];
+      return nd_kid(n, fronts, s, jr, jc < 0 ? (s ? n.cnK[1] : n.cnK[0]) : jc);
+    };
+    const auto own = [&](int a, int b) -> double {
+      const int64_t r = n.cell * C.Nt + a;
+      if (C.dflag[r])
+        return b < 0 ? C.dval[r] : (a == b ? 1. : 0.);
+      return (b < 0 ? C.rhs[r] : C.tt[r * C.Nt + b]) * scs[a];
+    };
+    constexpr int KM = (1 << NDKidBit) - 1;
+
+    for (int idx = tid; idx < NEM * NEM; idx += T)
+      {
+        const int i = idx % NEM, c = idx / NEM;
+        double    x = (i == c) ? 1. : 0.;
+        if (i < nE && c < nE)
+          x = LEAF ? own(e0[i], e0[c]) : kid(0, e0[i], e0[c]) + kid(1, e1[i], e1[c]);
+        LU[idx] = x;
+      }
+    __syncthreads();
+    if (warp == 0)
+      {
+        double v[RPL][NEM];
+        bool   used[RPL];
+        int    pos[RPL];
+#pragma unroll
+        for (int q = 0; q < RPL; ++q)
+          {
+            const int i = lane + 32 * q;
+            used[q]     = i >= NEM;
+            pos[q]      = i;
+#pragma unroll
+            for (int c = 0; c < NEM; ++c)
+              v[q][c] = LU[c * NEM + min(i, NEM - 1)];
+          }
+        bool bad = false;
+#pragma unroll
+        for (int j = 0; j < NEM; ++j)
+          {
+            if (j >= nE)
+              {
+                // the unit rows beyond nE keep their places
+                if (lane == j % 32)
+                  {
+                    dinv[j] = 1.;
+                    perm[j] = j;
+                  }
+                continue;
+              }
+            unsigned key = 0u;
+            int      qb  = 0;
+#pragma unroll
+            for (int q = 0; q < RPL; ++q)
+              if (!used[q] && lane + 32 * q < nE)
+                {
+                  const unsigned k = nd_pivot_key(v[q][j]);
+                  if (k > key)
+                    {
+                      key = k;
+                      qb  = q;
+                    }
+                }
+            const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
+            const int      src  = __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1;
+            const int      qs   = RPL > 1 ? __shfl_sync(0xffffffffu, qb, src) : 0;
+            const double   dl0 = v[0][j], dl1 = v[RPL - 1][j]; // values: a choice between elements would index
+            const double   d   = __shfl_sync(0xffffffffu, (RPL > 1 && qs) ? dl1 : dl0, src);
+            const double   hr   = (d != 0.) ? 1. / d : 0.;
+            bad |= !(fabs(d) > 0.) || !isfinite(d);
+            double l[RPL];
+#pragma unroll
+            for (int q = 0; q < RPL; ++q)
+              {
+                const bool me = lane == src && q == qs;
+                l[q]          = 0.;
+                if (me)
+                  {
+                    pos[q]  = j;
+                    used[q] = true;
+                    dinv[j] = hr;
+                    perm[j] = lane + 32 * q;
+                  }
+                else if (!used[q])
+                  {
+                    l[q]    = v[q][j] * hr;
+                    v[q][j] = l[q];
+                  }
+              }
+#pragma unroll
+            for (int c = j + 1; c < NEM; ++c)
+              {
+                const double pk0 = v[0][c], pk1 = v[RPL - 1][c];
+                const double pk  = __shfl_sync(0xffffffffu, (RPL > 1 && qs) ? pk1 : pk0, src);
+#pragma unroll
+                for (int q = 0; q < RPL; ++q)
+                  v[q][c] -= l[q] * pk;
+              }
+          }
+#pragma unroll
+        for (int q = 0; q < RPL; ++q)
+          if (lane + 32 * q < NEM)
+#pragma unroll
+            for (int c = 0; c < NEM; ++c)
+              LU[c * NEM + pos[q]] = v[q][c];
+        if (bad && lane == 0)
+          atomicExch(sing, 1);
+      }
+    else
+      {
+        const int t0 = tid - 32, TT = T - 32;
+        for (int idx = t0; idx < NEM * (nK + 1); idx += TT)
+          {
+            const int i = idx % NEM, c = idx / NEM;
+            double    x = 0.;
+            if (i < nE)
+              {
+                if (LEAF)
+                  x = own(e0[i], c < nK ? km[c] : -1);
+                else if (c == nK)
+                  x = kid(0, e0[i], -1) + kid(1, e1[i], -1);
+                else
+                  {
+                    const int s = km[c] >> NDKidBit;
+                    x           = kid(s, s ? e1[i] : e0[i], km[c] & KM);
+                  }
+              }
+            Bs[c * LDW + i] = x;
+          }
+        for (int idx = t0; idx < nK * NEM; idx += TT)
+          {
+            const int r = idx % nK, j = idx / nK;
+            double    x = 0.;
+            if (j < nE)
+              {
+                if (LEAF)
+                  x = own(km[r], e0[j]);
+                else
+                  {
+                    const int s = km[r] >> NDKidBit;
+                    x           = kid(s, km[r] & KM, s ? e1[j] : e0[j]);
+                  }
+              }
+            Ks[r * LDW + j] = -x;
+          }
+      }
+    __syncthreads();
+    // W, a thread per column
+    for (int c = tid; c <= nK; c += T)
+      {
+        double  x[NEM];
+        double *b = Bs + c * LDW;
+#pragma unroll
+        for (int i = 0; i < NEM; ++i)
+          x[i] = b[perm[i]];
+#pragma unroll
+        for (int r = 0; r < NEM; ++r)
+          {
+            // the factors are read where they are used: hoisted out of the
+            // column loop they would spill
+            asm volatile("" ::: "memory");
+#pragma unroll
+            for (int q = (r + 1) & ~1; q < NEM; q += 2)
+              {
+                const double2 lv = *reinterpret_cast<const double2 *>(LU + r * NEM + q);
+                if (q > r)
+                  x[q] -= lv.x * x[r];
+                x[q + 1] -= lv.y * x[r];
+              }
+          }
+#pragma unroll
+        for (int r = NEM - 1; r >= 0; --r)
+          {
+            asm volatile("" ::: "memory");
+            x[r] *= dinv[r];
+#pragma unroll
+            for (int q = 0; q < r; q += 2)
+              {
+                const double2 uv = *reinterpret_cast<const double2 *>(LU + r * NEM + q);
+                x[q] -= uv.x * x[r];
+                if (q + 1 < r)
+                  x[q + 1] -= uv.y * x[r];
+              }
+          }
+#pragma unroll
+        for (int i = 0; i < NEM; ++i)
+          b[i] = x[i];
+      }
+    __syncthreads();
+    double *Fv = fronts + n.koff;
+    for (int idx = tid; idx < nE * (nK + 1); idx += T)
+      {
+        const int i = idx % nE, c = idx / nE;
+        Fv[(int64_t)c * n.ld + i] = Bs[c * LDW + i];
+      }
+    // Schur complement
+    const int g = lane >> 2, tq = lane & 3;
+    const int rt = (nK + 15) / 16, ctn = (nK + 1 + 31) / 32;
+    for (int tile = warp; tile < rt * ctn; tile += T / 32)
+      {
+        const int r0 = (tile % rt) * 16, c0 = (tile / rt) * 32;
+        double    acc[2][4][2];
+        int       kr[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          {
+            const int r = r0 + i * 8 + g;
+            kr[i]       = r < nK ? km[r] : -1;
+          }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            {
+              const int c  = c0 + j * 8 + 2 * tq + e;
+              const int kc = c < nK ? km[c] : -1;
+#pragma unroll
+              for (int i = 0; i < 2; ++i)
+                {
+                  double x = 0.;
+                  if (kr[i] >= 0 && c <= nK)
+                    {
+                      if (LEAF)
+                        x = own(kr[i], kc);
+                      else if (c == nK)
+                        x = kid(kr[i] >> NDKidBit, kr[i] & KM, -1);
+                      else if ((kc >> NDKidBit) == (kr[i] >> NDKidBit))
+                        x = kid(kr[i] >> NDKidBit, kr[i] & KM, kc & KM);
+                    }
+                  acc[i][j][e] = x;
+                }
+            }
+#pragma unroll
+        for (int ks = 0; ks < NEM / 4; ++ks)
+          {
+            double a[2], b[4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              a[i] = Ks[min(r0 + i * 8 + g, nK - 1) * LDW + ks * 4 + tq];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              b[j] = Bs[min(c0 + j * 8 + g, nK) * LDW + ks * 4 + tq];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                dmma8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+          }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            {
+              const int c = c0 + j * 8 + 2 * tq + e;
+#pragma unroll
+              for (int i = 0; i < 2; ++i)
+                {
+                  const int r = r0 + i * 8 + g;
+                  if (r < nK && c <= nK)
+                    Fv[(int64_t)c * n.ld + n.nEp + r] = acc[i][j][e];
+                }
+            }
+      }
+  }
+
+  // ------------------------------------------------- E columns of the fronts
+  // F_EE and F_KE into the batch's scratch; CTA (some of the columns, node)
+  __global__ void __launch_bounds__(256)
+  nd_gather_e_kernel(const NDNode *nodes, const int32_t *maps, NDCells C, const double *fronts, double *ecols)
+  {
+    const NDNode  n = nodes[blockIdx.y];
+    const NDFront F{n, C, maps + n.map, fronts};
+    for (int j = blockIdx.x; j < n.nE; j += gridDim.x)
+      {
+        double *A = ecols + n.eoff + (int64_t)j * n.ld;
+        for (int i = threadIdx.x; i < n.ld; i += 256)
+          {
+            double x = 0.; // the pad rows stay zero
+            if (i < n.nE)
+              x = F.EE(i, j);
+            else if (i >= n.nEp && i - n.nEp < n.nK)
+              x = F.KE(i - n.nEp, j);
+            A[i] = x;
+          }
+      }
+  }
+
+  // [F_EK | r_E], rows in pivot order, into the E rows of the front; CTA
+  // (node, cb columns), staged in shared memory so that both sides are
+  // coalesced
+  __global__ void __launch_bounds__(256)
+  nd_gather_b_kernel(const NDNode *nodes, const int32_t *maps, NDCells C, const int32_t *perm_all, int cb,
+                     double *fronts)
+  {
+    extern __shared__ __align__(16) double sm[];
+    const NDNode n  = nodes[blockIdx.y];
+    const int    c0 = blockIdx.x * cb, nE = n.nE;
+    const int    nc = min(cb, n.nK + 1 - c0);
+    if (nc <= 0)
+      return;
+    const NDFront  F{n, C, maps + n.map, fronts};
+    const int32_t *perm = perm_all + n.poff;
+    for (int idx = threadIdx.x; idx < nc * nE; idx += 256)
+      sm[idx] = F.EK(idx % nE, c0 + idx / nE);
+    __syncthreads();
+    double *B = fronts + n.koff + (int64_t)c0 * n.ld;
+    for (int idx = threadIdx.x; idx < nc * n.nEp; idx += 256)
+      {
+        const int i = idx % n.nEp, c = idx / n.nEp;
+        B[(int64_t)c * n.ld + i] = i < nE ? sm[c * nE + perm[i]] : 0.; // the pad row stays zero
+      }
+  }
+
+  // -------------------------------------------------------------- dense LU
+  // Right-looking LU with partial pivoting of F_EE for all fronts of a batch,
+  // NDPanel columns per step, two launches per step.  Rows never move: every
+  // step works on the list of rows not chosen yet, and the factors are
+  // written in pivot order to their own array.
+  //
+  // nd_panel_kernel factorises a panel.  Each thread holds one row of it in
+  // registers; per column a warp max-reduction, one CTA barrier and, for the
+  // fronts whose rows need more than one CTA, one exchange of the C
+  // candidates through the distributed shared memory of a cluster of C CTAs.
+  // The kernel is a chain of NDPanel dependent column steps; the candidates'
+  // whole rows travel with their keys, so that a step has a single barrier.
+  constexpr int NDPanel   = 32;
+  constexpr int NDPanelT  = 512;           // threads per CTA at most
+  constexpr int NDPanelC  = 8;             // CTAs per cluster at most
+  constexpr int NDPanelLd = NDPanel + 4;   // shared row stride (= 4 mod 16)
+
+  template <int CL>
+  __global__ void __launch_bounds__(NDPanelT, 1)
+  nd_panel_kernel(const NDNode *nodes, int k0, const int32_t *ul_in, int32_t *ul_out, double *ecols,
+                  double *luf, int32_t *perm, double *tinv, int *sing)
+  {
+    namespace cg = cooperative_groups;
+    constexpr int       NW = NDPanelT / 32;
+    __shared__ __align__(16) double wrow[2][NW][NDPanel]; // candidate row per warp
+    __shared__ unsigned wkey[2][NW];
+    __shared__ int      wid[2][NW];
+    __shared__ __align__(16) double crow[2][CL][NDPanel]; // candidate row per CTA of the cluster
+    __shared__ unsigned ckey[2][CL];
+    __shared__ int      cid[2][CL];
+    __shared__ double   Ls[NDPanel][NDPanel + 1]; // pivot rows in pivot order
+    __shared__ int      ppos[NDPanel];            // their list positions
+    const NDNode       &n  = nodes[blockIdx.x / CL];
+    const int           nE = n.nE;
+    if (nE <= k0)
+      return; // every CTA of the cluster
+    const int rank = CL > 1 ? (int)(blockIdx.x % CL) : 0;
+    const int m = nE - k0, w = min(NDPanel, m);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x, nw = T >> 5;
+    const int t    = rank * T + tid; // position in the row list
+    const bool has = t < m;
+    const int  row = has ? (k0 ? ul_in[n.poff + t] : t) : 0;
+    double    *A   = ecols + n.eoff + (int64_t)k0 * n.ld;
+    double     v[NDPanel];
+#pragma unroll
+    for (int c = 0; c < NDPanel; ++c)
+      v[c] = (has && c < w) ? A[(int64_t)c * n.ld + row] : 0.;
+    bool used  = !has;
+    int  mypos = -1;
+    if (CL > 1)
+      cg::this_cluster().sync(); // every CTA of the cluster runs before its shared memory is written
+#pragma unroll
+    for (int j = 0; j < NDPanel; ++j)
+      if (j < w)
+        {
+          const int      buf  = j & 1;
+          const unsigned key  = used ? 0u : nd_pivot_key(v[j]);
+          const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
+          const int      src  = __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1;
+          if (lane == src)
+            {
+#pragma unroll
+              for (int c = 0; c < NDPanel; c += 2)
+                *reinterpret_cast<double2 *>(&wrow[buf][warp][c]) = make_double2(v[c], v[c + 1]);
+              wkey[buf][warp] = kmax;
+              wid[buf][warp]  = t;
+            }
+          __syncthreads();
+          const unsigned k2 = lane < nw ? wkey[buf][lane] : 0u;
+          const unsigned m2 = __reduce_max_sync(0xffffffffu, k2);
+          const int      ww = __ffs(__ballot_sync(0xffffffffu, lane < nw && k2 == m2)) - 1;
+          const double  *prow = wrow[buf][ww];
+          int            pid  = wid[buf][ww];
+          if (CL > 1)
+            {
+              cg::cluster_group cl = cg::this_cluster();
+              if (warp < CL)
+                {
+                  double *dst = cl.map_shared_rank(&crow[buf][rank][0], warp);
+                  dst[lane]   = prow[lane];
+                  if (lane == 0)
+                    {
+                      *cl.map_shared_rank(&ckey[buf][rank], warp) = m2;
+                      *cl.map_shared_rank(&cid[buf][rank], warp)  = pid;
+                    }
+                }
+              cl.sync();
+              const unsigned k3 = lane < CL ? ckey[buf][lane] : 0u;
+              const unsigned m3 = __reduce_max_sync(0xffffffffu, k3);
+              const int      cc = __ffs(__ballot_sync(0xffffffffu, lane < CL && k3 == m3)) - 1;
+              prow              = crow[buf][cc];
+              pid               = cid[buf][cc];
+            }
+          const double d  = prow[j];
+          const double hr = (d != 0.) ? 1. / d : 0.;
+          if (warp == 0)
+            {
+              if (rank == 0)
+                Ls[j][lane] = prow[lane];
+              if (lane == 0)
+                {
+                  ppos[j] = pid;
+                  if (rank == 0 && (!(fabs(d) > 0.) || !isfinite(d)))
+                    atomicExch(sing, 1);
+                }
+            }
+          if (!used)
+            {
+              if (t == pid)
+                {
+                  used  = true;
+                  mypos = j;
+                }
+              else
+                {
+                  const double l = v[j] * hr;
+                  v[j]           = l;
+#pragma unroll
+                  for (int c = j + 1; c < NDPanel; ++c)
+                    v[c] -= l * prow[c];
+                }
+            }
+        }
+    __syncthreads(); // Ls, ppos
+    const int ldl = n.nEp;
+    double   *LUF = luf + n.luoff + (int64_t)k0 * ldl + k0;
+    if (mypos >= 0)
+      perm[n.poff + k0 + mypos] = row;
+    else if (has)
+      {
+        int below = 0;
+#pragma unroll
+        for (int j = 0; j < NDPanel; ++j)
+          below += (j < w && ppos[j] < t) ? 1 : 0;
+        ul_out[n.poff + t - below] = row;
+#pragma unroll
+        for (int c = 0; c < NDPanel; ++c)
+          A[(int64_t)c * n.ld + row] = v[c]; // rows are left only when w == NDPanel
+      }
+    if (rank == 0)
+      {
+        for (int idx = tid; idx < w * w; idx += T)
+          LUF[(int64_t)(idx / w) * ldl + idx % w] = Ls[idx % w][idx / w];
+        // inverses of the unit lower and of the upper diagonal block (identity
+        // beyond w), a lane per column
+        if (warp < 2)
+          {
+            double x[NDPanel];
+            if (warp == 0)
+              {
+#pragma unroll
+                for (int r = 0; r < NDPanel; ++r)
+                  {
+                    double y = (r == lane) ? 1. : 0.;
+                    if (r < w)
+#pragma unroll
+                      for (int s = 0; s < r; ++s)
+                        y -= Ls[r][s] * x[s]; // x[s] = 0 for s < lane
+                    x[r] = y;
+                  }
+              }
+            else
+              {
+#pragma unroll
+                for (int r = NDPanel - 1; r >= 0; --r)
+                  {
+                    double y = (r == lane) ? 1. : 0.;
+                    if (r < w)
+                      {
+#pragma unroll
+                        for (int s = r + 1; s < NDPanel; ++s)
+                          if (s < w)
+                            y -= Ls[r][s] * x[s]; // x[s] = 0 for s > lane
+                        y /= Ls[r][r];
+                      }
+                    x[r] = y;
+                  }
+              }
+            double *out = tinv + n.tioff + ((int64_t)(k0 / NDPanel) * 2 + warp) * NDPanel * NDPanel;
+#pragma unroll
+            for (int r = 0; r < NDPanel; r += 2)
+              *reinterpret_cast<double2 *>(out + lane * NDPanel + r) = make_double2(x[r], x[r + 1]);
+          }
+      }
+    if (CL > 1)
+      cg::this_cluster().sync(); // no CTA leaves while its shared memory may still be written
+  }
+
+  __device__ __forceinline__ void
+  nd_cp_async8(double *dst, const double *src, bool valid)
+  {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const int      b = valid ? 8 : 0; // 0 source bytes: zero-filled
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(b));
+  }
+  __device__ __forceinline__ void
+  nd_cp_async16(double *dst, const double *src, int bytes)
+  {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes));
+  }
+  __device__ __forceinline__ void
+  nd_cp_commit()
+  {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  template <int N>
+  __device__ __forceinline__ void
+  nd_cp_wait()
+  {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+  }
+
+  // The step's trailing update: CTA (64 rows of the list x 64 columns) forms
+  // U12 = L11^-1 A[pivot rows] of its columns (the row tiles repeat it; the
+  // first one stores it in the factors) and subtracts L21 U12, both on the
+  // FP64 tensor path.
+  constexpr int NDUpd = 64;
+
+  __host__ __device__ constexpr size_t
+  nd_update_smem()
+  {
+    return (size_t)(3 * NDUpd + NDPanel) * NDPanelLd * sizeof(double);
+  }
+
+  __global__ void __launch_bounds__(128)
+  nd_update_kernel(const NDNode *nodes, int k0, int ctiles, const int32_t *ul, double *ecols, double *luf,
+                   const int32_t *perm, const double *tinv)
+  {
+    extern __shared__ __align__(16) double sm[];
+    __shared__ int rl[NDUpd];
+    double       (*Gs)[NDPanelLd] = reinterpret_cast<double (*)[NDPanelLd]>(sm); // [column][pivot row]
+    double       (*Us)[NDPanelLd] = Gs + NDUpd;                                  // [column][pivot row]
+    double       (*Ls)[NDPanelLd] = Us + NDUpd;                                  // [row][panel column]
+    double       (*Li)[NDPanelLd] = Ls + NDUpd;                                  // L11^-1, [column][row]
+    const NDNode  &n  = nodes[blockIdx.y];
+    const int      kn = k0 + NDPanel; // first trailing column
+    const int      m  = n.nE - kn;    // trailing rows and columns
+    const int      ct = blockIdx.x % ctiles, rt = blockIdx.x / ctiles;
+    if (ct * NDUpd >= m || rt * NDUpd >= m)
+      return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int c0 = kn + ct * NDUpd, nc = min(NDUpd, m - ct * NDUpd), nr = min(NDUpd, m - rt * NDUpd);
+    double   *A  = ecols + n.eoff;
+    const int64_t ld = n.ld;
+    if (tid < NDUpd)
+      rl[tid] = tid < nr ? ul[n.poff + rt * NDUpd + tid] : 0;
+    {
+      const int     k  = lane;
+      const double *gr = A + perm[n.poff + k0 + k];
+      for (int c = warp; c < NDUpd; c += 4)
+        nd_cp_async8(&Gs[c][k], gr + (c0 + min(c, nc - 1)) * ld, c < nc);
+      const double *ti = tinv + n.tioff + (int64_t)(k0 / NDPanel) * 2 * NDPanel * NDPanel;
+      for (int idx = tid; idx < NDPanel * NDPanel / 2; idx += 128)
+        nd_cp_async16(&Li[idx / 16][(idx % 16) * 2], ti + idx * 2, 16);
+    }
+    nd_cp_commit();
+    __syncthreads(); // rl
+    for (int idx = tid; idx < NDUpd * NDPanel; idx += 128)
+      {
+        const int r = idx % NDUpd, k = idx / NDUpd;
+        nd_cp_async8(&Ls[r][k], A + (k0 + k) * ld + rl[r], r < nr);
+      }
+    nd_cp_commit();
+    const int g = lane >> 2, q = lane & 3;
+    const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
+    double    acc[4][4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        {
+          const int c = wn + j * 8 + 2 * q + e;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            {
+              const int r  = wm + i * 8 + g;
+              acc[i][j][e] = (r < nr && c < nc) ? A[(c0 + c) * ld + rl[r]] : 0.;
+            }
+        }
+    nd_cp_wait<1>();
+    __syncthreads();
+    {
+      double u[4][2][2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          u[i][j][0] = u[i][j][1] = 0.;
+#pragma unroll
+      for (int ks = 0; ks < NDPanel / 4; ++ks)
+        {
+          double b[2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            b[j] = Gs[warp * 16 + j * 8 + g][ks * 4 + q];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            {
+              const double a = Li[ks * 4 + q][i * 8 + g];
+#pragma unroll
+              for (int j = 0; j < 2; ++j)
+                dmma8x8x4(u[i][j][0], u[i][j][1], a, b[j]);
+            }
+        }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            Us[warp * 16 + j * 8 + 2 * q + e][i * 8 + g] = u[i][j][e];
+    }
+    nd_cp_wait<0>();
+    __syncthreads();
+    if (rt == 0)
+      {
+        double *U = luf + n.luoff + (int64_t)c0 * n.nEp + k0;
+        for (int c = warp; c < nc; c += 4)
+          U[(int64_t)c * n.nEp + lane] = Us[c][lane];
+      }
+#pragma unroll
+    for (int ks = 0; ks < NDPanel / 4; ++ks)
+      {
+        double a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          a[i] = -Ls[wm + i * 8 + g][ks * 4 + q];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          b[j] = Us[wn + j * 8 + g][ks * 4 + q];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            dmma8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+      }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        {
+          const int c = wn + j * 8 + 2 * q + e;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            {
+              const int r = wm + i * 8 + g;
+              if (r < nr && c < nc)
+                A[(c0 + c) * ld + rl[r]] = acc[i][j][e];
+            }
+        }
+  }
+
+  // L below the diagonal blocks, from the rows' places into pivot order
+  __global__ void __launch_bounds__(256)
+  nd_lu_finish_kernel(const NDNode *nodes, const double *ecols, const int32_t *perm, double *luf)
+  {
+    const NDNode &n   = nodes[blockIdx.y];
+    const int     nE = n.nE, ldl = n.nEp;
+    const double *A = ecols + n.eoff;
+    double       *L = luf + n.luoff;
+    for (int c = blockIdx.x; c < (nE - 1) / NDPanel * NDPanel; c += gridDim.x)
+      for (int i = (c / NDPanel + 1) * NDPanel + threadIdx.x; i < nE; i += 256)
+        L[(int64_t)c * ldl + i] = A[(int64_t)c * n.ld + perm[n.poff + i]];
+  }
+
+  // The fronts beyond the panel kernel's rows: LU by cuSOLVER in place of
+  // F_EE; its row swaps (1-based) turned into the pivot order, the factors
+  // copied, the diagonal blocks inverted.  One front per launch.
+  __global__ void
+  nd_lib_perm_kernel(const NDNode *node, const int *ipiv, const int *info, int32_t *perm, int *sing)
+  {
+    int32_t *pm = perm + node->poff;
+    for (int i = threadIdx.x; i < node->nE; i += blockDim.x)
+      pm[i] = i;
+    __syncthreads();
+    if (threadIdx.x)
+      return;
+    if (*info)
+      atomicExch(sing, 1);
+    for (int j = 0; j < node->nE; ++j)
+      {
+        const int k = ipiv[j] - 1, x = pm[j];
+        pm[j]       = pm[k];
+        pm[k]       = x;
+      }
+  }
+
+  __global__ void __launch_bounds__(256)
+  nd_lib_copy_kernel(const NDNode *node, const double *ecols, double *luf)
+  {
+    const NDNode &n = *node;
+    for (int c = blockIdx.x; c < n.nE; c += gridDim.x)
+      for (int i = threadIdx.x; i < n.nE; i += 256)
+        luf[n.luoff + (int64_t)c * n.nEp + i] = ecols[n.eoff + (int64_t)c * n.ld + i];
+  }
+
+  __global__ void __launch_bounds__(64)
+  nd_lib_inverse_kernel(const NDNode *node, const double *luf, double *tinv)
+  {
+    __shared__ double S[NDPanel][NDPanel + 1];
+    const NDNode &n  = *node;
+    const int     r0 = blockIdx.x * NDPanel, w = min(NDPanel, n.nE - r0);
+    const int     lane = threadIdx.x & 31, which = threadIdx.x >> 5;
+    for (int idx = threadIdx.x; idx < NDPanel * NDPanel; idx += 64)
+      {
+        const int r = idx % NDPanel, c = idx / NDPanel;
+        S[r][c] = (r < w && c < w) ? luf[n.luoff + (int64_t)(r0 + c) * n.nEp + r0 + r] : (r == c ? 1. : 0.);
+      }
+    __syncthreads();
+    double x[NDPanel];
+    if (which == 0)
+      {
+#pragma unroll
+        for (int r = 0; r < NDPanel; ++r)
+          {
+            double y = (r == lane) ? 1. : 0.;
+#pragma unroll
+            for (int s = 0; s < r; ++s)
+              y -= S[r][s] * x[s];
+            x[r] = y;
+          }
+      }
+    else
+      {
+#pragma unroll
+        for (int r = NDPanel - 1; r >= 0; --r)
+          {
+            double y = (r == lane) ? 1. : 0.;
+#pragma unroll
+            for (int s = r + 1; s < NDPanel; ++s)
+              y -= S[r][s] * x[s];
+            x[r] = y / S[r][r];
+          }
+      }
+    double *out = tinv + n.tioff + ((int64_t)blockIdx.x * 2 + which) * NDPanel * NDPanel;
+    for (int r = 0; r < NDPanel; ++r)
+      out[lane * NDPanel + r] = x[r];
+  }
+
+  // ------------------------------------------------------ triangular solves
+  // W_b = U_bb^-1 L_bb^-1 B_b for the rows [b0, b0 + bs) of the fronts
+  // (dir bit 0: L, bit 1: U), in place.  CTA (32 columns, front): the whole
+  // column tile stays in shared memory for both sweeps; the 32 x 32 blocks of
+  // the factors stream through a ring of cp.async stages, the diagonal blocks
+  // as their inverses, all products on the FP64 tensor path.  Bound by the
+  // factors' L2 reads and the tensor path; one read and one write of B.
+  constexpr int NDSolveCols   = 32;
+  constexpr int NDSolveStages = 4;
+
+  __host__ __device__ inline size_t
+  nd_solve_smem(int bs)
+  {
+    const int rows = (bs + NDPanel - 1) / NDPanel * NDPanel;
+    return ((size_t)NDSolveCols * (rows + 4) + (size_t)NDSolveStages * NDPanel * NDPanelLd) * sizeof(double);
+  }
+
+  __global__ void __launch_bounds__(256)
+  nd_solve_kernel(const NDNode *nodes, int b0, int bs, int dir, const double *luf, const double *tinv,
+                  double *fronts)
+  {
+    extern __shared__ __align__(16) double sm[];
+    const NDNode &n  = nodes[blockIdx.y];
+    const int     c0 = blockIdx.x * NDSolveCols, nc = min(NDSolveCols, n.nK + 1 - c0);
+    const int     nr = min(bs, n.nE - b0);
+    if (nc <= 0 || nr <= 0)
+      return;
+    const int     nblk = (nr + NDPanel - 1) / NDPanel;
+    const int     ldb  = (bs + NDPanel - 1) / NDPanel * NDPanel + 4;
+    double       *Bs   = sm;                                   // [column][row]
+    double       *Ts   = sm + (size_t)NDSolveCols * ldb;       // stages of [column][row] blocks
+    const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int     g = lane >> 2, q = lane & 3;
+    const int     mt = warp & 3, nt = (warp >> 2) * 2;
+    double       *B  = fronts + n.koff + (int64_t)c0 * n.ld + b0;
+    const double *LU = luf + n.luoff + (int64_t)b0 * n.nEp + b0;
+    const double *TI = tinv + n.tioff + (int64_t)(b0 / NDPanel) * 2 * NDPanel * NDPanel;
+    const int     ldl = n.nEp;
+    for (int c = warp; c < NDSolveCols; c += 8)
+      for (int r = lane; r < nblk * NDPanel; r += 32)
+        Bs[c * ldb + r] = (c < nc && r < nr) ? B[(int64_t)c * n.ld + r] : 0.;
+
+    // the blocks in the order of use: (sweep, block row i, block column j);
+    // j == i stands for the diagonal block's inverse, the last of its row
+    struct It
+    {
+      int d, i, j;
+    };
+    const auto first = [&](int d) { return d == 0 ? It{0, 0, 0} : It{1, nblk - 1, nblk - 1}; };
+    const auto next  = [&](It t) {
+      // forward rows: j = 0 .. i; backward rows: j = nblk - 1 .. i
+      if (t.d == 0)
+        {
+          if (t.j < t.i)
+            return It{0, t.i, t.j + 1};
+          if (t.i + 1 < nblk)
+            return It{0, t.i + 1, 0};
+          return (dir & 2) ? first(1) : It{2, 0, 0};
+        }
+      if (t.j > t.i)
+        return It{1, t.i, t.j - 1};
+      if (t.i > 0)
+        return It{1, t.i - 1, nblk - 1};
+      return It{2, 0, 0};
+    };
+    const auto issue = [&](It t, int stage) {
+      if (t.d < 2)
+        {
+          double *dst = Ts + (size_t)stage * NDPanel * NDPanelLd;
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            {
+              const int idx = tid + 256 * h, r = (idx % 16) * 2, k = idx / 16;
+              if (t.j == t.i)
+                nd_cp_async16(dst + k * NDPanelLd + r,
+                              TI + ((int64_t)t.i * 2 + t.d) * NDPanel * NDPanel + k * NDPanel + r, 16);
+              else
+                {
+                  const int rr = t.i * NDPanel + r, kk = t.j * NDPanel + k;
+                  const int bytes = kk < nr ? 8 * max(0, min(2, nr - rr)) : 0;
+                  nd_cp_async16(dst + k * NDPanelLd + r, bytes ? LU + (int64_t)kk * ldl + rr : LU, bytes);
+                }
+            }
+        }
+      nd_cp_commit();
+    };
+    It p = first((dir & 1) ? 0 : 1), t = p;
+#pragma unroll
+    for (int s = 0; s < NDSolveStages - 1; ++s)
+      {
+        issue(p, s);
+        if (p.d < 2)
+          p = next(p);
+      }
+    double acc[2][2] = {};
+    bool   fresh     = true; // the row's accumulators are not loaded yet
+    for (int it = 0; t.d < 2; ++it)
+      {
+        nd_cp_wait<NDSolveStages - 2>();
+        __syncthreads();
+        issue(p, (it + NDSolveStages - 1) % NDSolveStages);
+        if (p.d < 2)
+          p = next(p);
+        const double *A = Ts + (size_t)(it % NDSolveStages) * NDPanel * NDPanelLd;
+        const int     row = t.i * NDPanel + mt * 8 + g;
+        if (fresh && t.j != t.i)
+          {
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                acc[j][e] = Bs[((nt + j) * 8 + 2 * q + e) * ldb + row];
+            fresh = false;
+          }
+        if (t.j != t.i)
+          {
+#pragma unroll
+            for (int ks = 0; ks < NDPanel / 4; ++ks)
+              {
+                const double a = -A[(ks * 4 + q) * NDPanelLd + mt * 8 + g];
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                  dmma8x8x4(acc[j][0], acc[j][1], a, Bs[((nt + j) * 8 + g) * ldb + t.j * NDPanel + ks * 4 + q]);
+              }
+          }
+        else
+          {
+            if (!fresh)
+              {
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                  for (int e = 0; e < 2; ++e)
+                    Bs[((nt + j) * 8 + 2 * q + e) * ldb + row] = acc[j][e];
+                __syncthreads();
+              }
+            double o[2][2] = {};
+#pragma unroll
+            for (int ks = 0; ks < NDPanel / 4; ++ks)
+              {
+                const double a = A[(ks * 4 + q) * NDPanelLd + mt * 8 + g];
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                  dmma8x8x4(o[j][0], o[j][1], a, Bs[((nt + j) * 8 + g) * ldb + t.i * NDPanel + ks * 4 + q]);
+              }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                Bs[((nt + j) * 8 + 2 * q + e) * ldb + row] = o[j][e];
+            fresh = true;
+          }
+        t = next(t);
+      }
+    nd_cp_wait<0>();
+    __syncthreads();
+    for (int c = warp; c < nc; c += 8)
+      for (int r = lane; r < nr; r += 32)
+        B[(int64_t)c * n.ld + r] = Bs[c * ldb + r];
+  }
+
+  // ------------------------------------------------------------ C -= A B
+  // 64 x 64 tiles of C, 128 threads (2 x 2 warps of 32 x 32), 16-deep stages
+  // of A and B through cp.async.
+  // SCHUR: F_KK - F_KE W with the front's entries (the children's) as the
+  // initial accumulators, stored once, the right-hand-side column included.
+  // Otherwise: rows [r0, r0 + mr) of the E rows of the fronts minus the
+  // factors' block times the solved rows [b0, b0 + bs) (blocked triangular
+  // solves of the fronts whose columns do not fit in shared memory).
+  constexpr int NDGM = 64, NDGN = 64, NDGK = 16;
+  constexpr int NDGLA = NDGM + 4; // As[k][m] row stride (= 4 mod 16)
+  constexpr int NDGLB = NDGK + 4; // Bs[n][k] row stride
+  constexpr int NDGStages = 3;
+
+  __host__ __device__ constexpr size_t
+  nd_gemm_smem()
+  {
+    return (size_t)NDGStages * (NDGK * NDGLA + NDGN * NDGLB) * sizeof(double);
+  }
+
+  template <bool SCHUR>
+  __global__ void __launch_bounds__(128)
+  nd_gemm_kernel(const NDNode *nodes, const int32_t *maps, NDCells Cc, int tiles_m, int r0, int mr, int b0, int bs,
+                 const double *ecols, const double *luf, double *fronts)
+  {
+    extern __shared__ __align__(16) double sm[];
+    const NDNode  n  = nodes[blockIdx.y];
+    const int     m0 = (blockIdx.x % tiles_m) * NDGM, n0 = (blockIdx.x / tiles_m) * NDGN;
+    const int     m  = SCHUR ? n.nK : min(mr, n.nE - r0);
+    const int     nn = n.nK + 1;
+    const int     k  = SCHUR ? n.nE : min(bs, n.nE - b0);
+    if (m0 >= m || n0 >= nn || k <= 0)
+      return;
+    const int64_t lda = SCHUR ? n.ld : n.nEp;
+    const double *A   = SCHUR ? ecols + n.eoff + n.nEp : luf + n.luoff + (int64_t)b0 * n.nEp + r0;
+    double       *F   = fronts + n.koff;
+    const double *Bm  = F + (SCHUR ? 0 : b0);
+    double       *Cm  = F + (SCHUR ? n.nEp : r0);
+    const int     tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int     wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
+    const int     nchunk = (k + NDGK - 1) / NDGK;
+    const int     g = lane >> 2, q = lane & 3;
+
+    const auto As = [&](int st) { return sm + (size_t)st * (NDGK * NDGLA + NDGN * NDGLB); };
+    const auto issue = [&](int chunk, int st) {
+      if (chunk < nchunk)
+        {
+          double   *a = As(st), *b = a + NDGK * NDGLA;
+          const int k0 = chunk * NDGK;
+#pragma unroll
+          for (int h = 0; h < NDGM * NDGK / 2 / 128; ++h)
+            {
+              const int  idx = tid + 128 * h, mm = (idx % (NDGM / 2)) * 2, kk = idx / (NDGM / 2);
+              const bool ok = m0 + mm < m && k0 + kk < k; // rows are padded to even
+              nd_cp_async16(a + kk * NDGLA + mm, ok ? A + (k0 + kk) * lda + m0 + mm : A, ok ? 16 : 0);
+            }
+#pragma unroll
+          for (int h = 0; h < NDGN * NDGK / 2 / 128; ++h)
+            {
+              const int idx = tid + 128 * h, kk = (idx % (NDGK / 2)) * 2, c = idx / (NDGK / 2);
+              const int bytes = n0 + c < nn ? 8 * max(0, min(2, k - k0 - kk)) : 0;
+              nd_cp_async16(b + c * NDGLB + kk, bytes ? Bm + (int64_t)(n0 + c) * n.ld + k0 + kk : Bm, bytes);
+            }
+        }
+      nd_cp_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < NDGStages - 1; ++s)
+      issue(s, s);
+    double acc[4][4][2];
+    if (SCHUR)
+      {
+        const NDFront  F_{n, Cc, maps + n.map, fronts};
+        const int32_t *km = maps + n.map + 2 * n.nE;
+        constexpr int  KM = (1 << NDKidBit) - 1;
+        int            kr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          {
+            const int r = m0 + wm + i * 8 + g;
+            kr[i]       = (n.cell < 0 && r < m) ? km[r] : -1;
+          }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            {
+              const int c  = n0 + wn + j * 8 + 2 * q + e;
+              const int kc = (n.cell < 0 && c < n.nK) ? km[c] : -1;
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                {
+                  const int r = m0 + wm + i * 8 + g;
+                  double    x = 0.;
+                  if (r < m && c < nn)
+                    {
+                      if (n.cell >= 0)
+                        x = F_.KK(r, c);
+                      else
+                        {
+                          const int s = kr[i] >> NDKidBit;
+                          if (c == n.nK)
+                            x = nd_kid(n, fronts, s, kr[i] & KM, s ? n.cnK[1] : n.cnK[0]);
+                          else if ((kc >> NDKidBit) == s)
+                            x = nd_kid(n, fronts, s, kr[i] & KM, kc & KM);
+                        }
+                    }
+                  acc[i][j][e] = x;
+                }
+            }
+      }
+    else
+      {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            {
+              const int c = n0 + wn + j * 8 + 2 * q + e;
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                {
+                  const int r  = m0 + wm + i * 8 + g;
+                  acc[i][j][e] = (r < m && c < nn) ? Cm[(int64_t)c * n.ld + r] : 0.;
+                }
+            }
+      }
+    for (int c = 0; c < nchunk; ++c)
+      {
+        nd_cp_wait<NDGStages - 2>();
+        __syncthreads();
+        issue(c + NDGStages - 1, (c + NDGStages - 1) % NDGStages);
+        const double *a_s = As(c % NDGStages), *b_s = a_s + NDGK * NDGLA;
+#pragma unroll
+        for (int ks = 0; ks < NDGK / 4; ++ks)
+          {
+            double a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              a[i] = -a_s[(ks * 4 + q) * NDGLA + wm + i * 8 + g];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              b[j] = b_s[(wn + j * 8 + g) * NDGLB + ks * 4 + q];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                dmma8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+          }
+      }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        {
+          const int c = n0 + wn + j * 8 + 2 * q + e;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            {
+              const int r = m0 + wm + i * 8 + g;
+              if (r < m && c < nn)
+                Cm[(int64_t)c * n.ld + r] = acc[i][j][e];
+            }
+        }
+  }
+
+  // ------------------------------------------------------ back substitution
+  // x_E = y_E - W x_K for every node of a batch.  CTA (node, block of R
+  // eliminated rows) of R x S threads: thread (row t % R, slice t / R) sums
+  // the terms k = slice, slice + S, ... of W x_K (for one k the R rows are
+  // consecutive in memory), and the S partial sums of a row are added in
+  // shared memory.  Short dependency chains: the top fronts have few rows per
+  // node and thousands of kept dofs.
+  __global__ void
+  nd_backsolve_kernel(int R, const NDNode *nodes, const int32_t *fdofs, const double *fronts, double *x)
+  {
+    extern __shared__ __align__(16) double sm[];
+    const NDNode &n  = nodes[blockIdx.x];
+    const int     nE = n.nE, nK = n.nK;
+    if ((int)blockIdx.y * R >= nE)
+      return;
+    const int      S    = blockDim.x / R;
+    double        *xk   = sm;
+    double        *part = sm + nK;
+    const int32_t *dl   = fdofs + n.doff;
+    for (int k = threadIdx.x; k < nK; k += blockDim.x)
+      xk[k] = x[dl[nE + k]];
+    __syncthreads();
+    const double *Fv = fronts + n.koff;
+    const int     t = threadIdx.x, il = t % R, sl = t / R;
+    const int     i = blockIdx.y * R + il;
+    if (sl < S)
+      {
+        double v = 0.;
+        if (i < nE)
+          for (int k = sl; k < nK; k += S)
+            v += Fv[(int64_t)k * n.ld + i] * xk[k];
+        part[sl * R + il] = v;
+      }
+    __syncthreads();
+    if (t < R && i < nE)
+      {
+        double v = Fv[(int64_t)nK * n.ld + i];
+        for (int s = 0; s < S; ++s)
+          v -= part[s * R + t];
+        x[dl[i]] = v;
+      }
+  }
+} // namespace ddhdg
