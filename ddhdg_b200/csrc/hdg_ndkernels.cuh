@@ -171,10 +171,10 @@ namespace ddhdg
 
   // ------------------------------------------------------------ small fronts
   // nE <= NEM <= 36: the whole elimination of a front in one CTA.
-  // - F_EE goes into the registers of warp 0 (one row per lane, two for
-  //   NEM > 32; unit rows beyond nE): LU with virtual partial pivoting, the
-  //   pivot search one warp max-reduction, the pivot row broadcast by
-  //   shuffles, no barrier; the other warps stage [F_EK | r_E] and -F_KE.
+  // - F_EE goes into the registers of one warp (two for NEM > 32), a row per
+  //   lane: LU with virtual partial pivoting, the pivot search one warp
+  //   max-reduction, the pivot row broadcast through shared memory; the other
+  //   warps stage [F_EK | r_E] and -F_KE.
   // - W: a thread per column, its nE entries in registers, the factors
   //   broadcast from shared memory; no barrier between its steps.
   // - F_KK - F_KE W: 16 x 32 warp tiles on the FP64 tensor path with the
@@ -191,189 +191,199 @@ namespace ddhdg
   constexpr int NDSmallE = 36;
 
   __host__ __device__ inline size_t
-  nd_small_smem(int NEM, int nK, int Nt)
+  nd_small_smem(int NEM, int nK)
   {
     // rows of Bs / Ks hold NEM doubles: NEM = 4 or 12 (mod 16), so the
     // tensor-path fragments read distinct banks
-    return ((size_t)NEM * NEM + NEM + (size_t)(2 * nK + 1) * NEM + 2 * (size_t)Nt) * sizeof(double) +
-           ((size_t)nK + 3 * NEM) * sizeof(int);
+    return ((size_t)NEM * NEM + NEM + (size_t)(2 * nK + 1) * NEM + 2 * (size_t)nK + 4 * NEM) * sizeof(double) +
+           ((size_t)nK * 2 + 4 * NEM) * sizeof(int);
   }
 
   template <int NEM, bool LEAF>
-  __global__ void __launch_bounds__(256)
+  __global__ void __launch_bounds__(NEM > 28 ? 512 : 256, NEM <= 12 ? 4 : NEM <= 20 ? 3 : NEM <= 28 ? 2 : 1)
   nd_small_kernel(const NDNode *nodes, const int32_t *maps, NDCells C, int nKmax, int *sing, double *fronts)
   {
     extern __shared__ __align__(16) double sm[];
     constexpr int LDW = NEM;
-    constexpr int RPL = NEM > 32 ? 2 : 1;
+    constexpr int NLW = NEM > 32 ? 2 : 1; // warps of the LU, a row per lane
+    __shared__ __align__(16) double prow_s[2][NLW][NEM];
+    __shared__ double   phr_s[2][NLW];
+    __shared__ unsigned pkey_s[2][NLW];
+    __shared__ int      pid_s[2][NLW];
     const NDNode  n   = nodes[blockIdx.x];
     const int     nE = n.nE, nK = n.nK;
-    double       *LU   = sm;                       // factors, [column][pivot order]
-    double       *dinv = LU + NEM * NEM;           // 1 / U_jj
-    double       *Bs   = dinv + NEM;               // [column of K, r][E row]
-    double       *Ks   = Bs + (nKmax + 1) * LDW;   // -F_KE: [K row][E column]
-    double       *scs  = Ks + nKmax * LDW;         // row scales of cells read directly
-    int          *km   = reinterpret_cast<int *>(scs + 2 * C.Nt);
-    int          *e0   = km + nKmax;
-    int          *e1   = e0 + NEM;
-    int          *perm = e1 + NEM;
-    const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
+    double       *LU   = sm;                     // factors, [column][pivot order]
+    double       *dinv = LU + NEM * NEM;         // 1 / U_jj
+    double       *Bs   = dinv + NEM;             // [column of K, r][E row]
+    double       *Ks   = Bs + (nKmax + 1) * LDW; // -F_KE: [K row][E column]
+    // Every position of the front as a row and as a column of the child (or
+    // cell) that holds it: an entry is rs * rp[column offset].  A K position
+    // belongs to one child, an E position to both.
+    double        *krs  = Ks + nKmax * LDW;                    // row scale
+    double        *ers  = krs + nKmax;                         // [2][NEM]
+    const double **krp  = (const double **)(ers + 2 * NEM);    // row pointer
+    const double **erp  = krp + nKmax;                         // [2][NEM]
+    int           *kco  = reinterpret_cast<int *>(erp + 2 * NEM); // column offset
+    int           *kid  = kco + nKmax;                         // child of a K position
+    int           *eco  = kid + nKmax;                         // [2][NEM]
+    int           *perm = eco + 2 * NEM;
+    const int      tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
     const int32_t *map = maps + n.map;
-    if (LEAF)
-      {
-        for (int i = tid; i < nE; i += T)
-          e0[i] = map[i];
-        for (int i = tid; i < nK; i += T)
-          km[i] = map[nE + i];
-        for (int a = tid; a < C.Nt; a += T)
-          scs[a] = nd_cell_scale(C, n.cell, a);
-      }
-    else
-      {
-        for (int i = tid; i < nE; i += T)
-          {
-            e0[i] = map[i];
-            e1[i] = map[nE + i];
-          }
-        for (int i = tid; i < nK; i += T)
-          km[i] = map[2 * nE + i];
-#pragma unroll
-        for (int s = 0; s < 2; ++s)
-          if (n.ccell[s] >= 0)
-            for (int a = tid; a < C.Nt; a += T)
-              scs[s * C.Nt + a] = nd_cell_scale(C, n.ccell[s], a);
-      }
-    __syncthreads();
-    // entries by local indices of child s (or of the node's own cell);
-    // column -1 is the right-hand side
-    const auto kid = [&](int s, int jr, int jc) -> double {
-      const int64_t cell = s ? n.ccell[1] : n.ccell[0];
+    constexpr int  KM  = (1 << NDKidBit) - 1;
+    // row jr, column offset jc of child s; raw cells carry the row scaling,
+    // their Dirichlet rows are identity rows (scale 0, the diagonal apart)
+    const auto place = [&](int s, int j, const double *&rp, double &rs, int &co) {
+      const int64_t cell = LEAF ? n.cell : (s ? n.ccell[1] : n.ccell[0]);
       if (cell >= 0)
-        return (jc < 0 ? C.rhs[cell * C.Nt + jr] : C.tt[(cell * C.Nt + jr) * (int64_t)C.Nt + jc]) *
-               scs[s * C.Nt + jr];
-      return nd_kid(n, fronts, s, jr, jc < 0 ? (s ? n.cnK[1] : n.cnK[0]) : jc);
+        {
+          rp = C.tt + (cell * C.Nt + j) * (int64_t)C.Nt;
+          rs = C.dflag[cell * C.Nt + j] ? 0. : nd_cell_scale(C, cell, j);
+          co = j;
+        }
+      else
+        {
+          rp = fronts + (s ? n.coff[1] : n.coff[0]) + (s ? n.cEp[1] : n.cEp[0]) + j;
+          rs = 1.;
+          co = j * (s ? n.cld[1] : n.cld[0]);
+        }
     };
-    const auto own = [&](int a, int b) -> double {
-      const int64_t r = n.cell * C.Nt + a;
-      if (C.dflag[r])
-        return b < 0 ? C.dval[r] : (a == b ? 1. : 0.);
-      return (b < 0 ? C.rhs[r] : C.tt[r * C.Nt + b]) * scs[a];
+    for (int i = tid; i < nE; i += T)
+#pragma unroll
+      for (int s = 0; s < (LEAF ? 1 : 2); ++s)
+        place(s, map[LEAF ? i : s * nE + i], erp[s * NEM + i], ers[s * NEM + i], eco[s * NEM + i]);
+    for (int i = tid; i < nK; i += T)
+      {
+        const int k = LEAF ? map[nE + i] : map[2 * nE + i], s = LEAF ? 0 : k >> NDKidBit;
+        place(s, k & KM, krp[i], krs[i], kco[i]);
+        kid[i] = s;
+      }
+    const bool cells = LEAF || n.ccell[0] >= 0 || n.ccell[1] >= 0;
+    __syncthreads();
+    // entry of a row (pointer, scale, column offset of its own position)
+    const auto entry = [&](const double *rp, double rs, int own, int co) -> double {
+      if (cells && rs == 0.)
+        return own == co ? 1. : 0.;
+      return rs * rp[co];
     };
-    constexpr int KM = (1 << NDKidBit) - 1;
-
+    // right-hand side of a row of child s
+    const auto rhs = [&](int s, const double *rp, double rs, int own) -> double {
+      const int64_t cell = LEAF ? n.cell : (s ? n.ccell[1] : n.ccell[0]);
+      if (cell >= 0)
+        {
+          const int64_t r = cell * C.Nt + own;
+          return rs == 0. ? C.dval[r] : rs * C.rhs[r];
+        }
+      return rp[(int64_t)(s ? n.cnK[1] : n.cnK[0]) * (s ? n.cld[1] : n.cld[0])];
+    };
     for (int idx = tid; idx < NEM * NEM; idx += T)
       {
         const int i = idx % NEM, c = idx / NEM;
         double    x = (i == c) ? 1. : 0.;
         if (i < nE && c < nE)
-          x = LEAF ? own(e0[i], e0[c]) : kid(0, e0[i], e0[c]) + kid(1, e1[i], e1[c]);
+          {
+            x = entry(erp[i], ers[i], eco[i], eco[c]);
+            if (!LEAF)
+              x += entry(erp[NEM + i], ers[NEM + i], eco[NEM + i], eco[NEM + c]);
+          }
         LU[idx] = x;
       }
     __syncthreads();
-    if (warp == 0)
+    if (warp < NLW)
       {
-        double v[RPL][NEM];
-        bool   used[RPL];
-        int    pos[RPL];
+        // rolled steps (the instruction cache holds the body): the row is
+        // rotated by one register per step, the current column in v[0]
+        double v[NEM];
 #pragma unroll
-        for (int q = 0; q < RPL; ++q)
+        for (int c = 0; c < NEM; ++c)
+          v[c] = LU[c * NEM + min(tid, NEM - 1)];
+        bool used = tid >= nE, bad = false;
+        int  pos  = -1;
+#pragma unroll 1
+        for (int j = 0; j < nE; ++j)
           {
-            const int i = lane + 32 * q;
-            used[q]     = i >= NEM;
-            pos[q]      = i;
-#pragma unroll
-            for (int c = 0; c < NEM; ++c)
-              v[q][c] = LU[c * NEM + min(i, NEM - 1)];
-          }
-        bool bad = false;
-#pragma unroll
-        for (int j = 0; j < NEM; ++j)
-          {
-            if (j >= nE)
-              {
-                // the unit rows beyond nE keep their places
-                if (lane == j % 32)
-                  {
-                    dinv[j] = 1.;
-                    perm[j] = j;
-                  }
-                continue;
-              }
-            unsigned key = 0u;
-            int      qb  = 0;
-#pragma unroll
-            for (int q = 0; q < RPL; ++q)
-              if (!used[q] && lane + 32 * q < nE)
-                {
-                  const unsigned k = nd_pivot_key(v[q][j]);
-                  if (k > key)
-                    {
-                      key = k;
-                      qb  = q;
-                    }
-                }
+            const int      buf  = j & 1;
+            const double   x0   = v[0];
+            const unsigned key  = used ? 0u : nd_pivot_key(x0);
+            const double   hx   = (x0 != 0.) ? 1. / x0 : 0.; // overlaps the reduction
             const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
             const int      src  = __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1;
-            const int      qs   = RPL > 1 ? __shfl_sync(0xffffffffu, qb, src) : 0;
-            const double   dl0 = v[0][j], dl1 = v[RPL - 1][j]; // values: a choice between elements would index
-            const double   d   = __shfl_sync(0xffffffffu, (RPL > 1 && qs) ? dl1 : dl0, src);
-            const double   hr   = (d != 0.) ? 1. / d : 0.;
-            bad |= !(fabs(d) > 0.) || !isfinite(d);
-            double l[RPL];
-#pragma unroll
-            for (int q = 0; q < RPL; ++q)
+            if (lane == src)
               {
-                const bool me = lane == src && q == qs;
-                l[q]          = 0.;
-                if (me)
-                  {
-                    pos[q]  = j;
-                    used[q] = true;
-                    dinv[j] = hr;
-                    perm[j] = lane + 32 * q;
-                  }
-                else if (!used[q])
-                  {
-                    l[q]    = v[q][j] * hr;
-                    v[q][j] = l[q];
-                  }
+                // finished columns, at the end, are published as zeros
+                double2 *dst = reinterpret_cast<double2 *>(prow_s[buf][warp]);
+#pragma unroll
+                for (int k = 0; k < NEM; k += 2)
+                  dst[k / 2] = make_double2(k < NEM - j ? v[k] : 0., k + 1 < NEM - j ? v[k + 1] : 0.);
+                phr_s[buf][warp]  = hx;
+                pkey_s[buf][warp] = kmax;
+                pid_s[buf][warp]  = tid;
               }
+            if (NLW > 1)
+              asm volatile("bar.sync 1, 64;" ::: "memory");
+            else
+              __syncwarp();
+            const int     ww   = (NLW > 1 && pkey_s[buf][NLW - 1] > pkey_s[buf][0]) ? NLW - 1 : 0;
+            const double *prow = prow_s[buf][ww];
+            const double  hr   = phr_s[buf][ww];
+            const int     pid  = pid_s[buf][ww];
+            const bool    me   = tid == pid;
+            const double  l    = (used || me) ? 0. : x0 * hr;
 #pragma unroll
-            for (int c = j + 1; c < NEM; ++c)
+            for (int k = 1; k < NEM; ++k)
+              v[k - 1] = v[k] - l * prow[k];
+            v[NEM - 1] = (used || me) ? x0 : l;
+            if (me)
               {
-                const double pk0 = v[0][c], pk1 = v[RPL - 1][c];
-                const double pk  = __shfl_sync(0xffffffffu, (RPL > 1 && qs) ? pk1 : pk0, src);
-#pragma unroll
-                for (int q = 0; q < RPL; ++q)
-                  v[q][c] -= l[q] * pk;
+                used    = true;
+                pos     = j;
+                dinv[j] = hr;
+                perm[j] = tid;
+                bad |= !(fabs(x0) > 0.) || !isfinite(x0);
               }
           }
+#pragma unroll 1
+        for (int j = nE; j < NEM; ++j)
+          {
+            // the unit rows and columns beyond nE keep their places
+            const double x0 = v[0];
 #pragma unroll
-        for (int q = 0; q < RPL; ++q)
-          if (lane + 32 * q < NEM)
+            for (int k = 1; k < NEM; ++k)
+              v[k - 1] = v[k];
+            v[NEM - 1] = x0;
+            if (tid == 0)
+              {
+                dinv[j] = 1.;
+                perm[j] = j;
+              }
+          }
+        if (pos >= 0)
+          {
 #pragma unroll
             for (int c = 0; c < NEM; ++c)
-              LU[c * NEM + pos[q]] = v[q][c];
-        if (bad && lane == 0)
+              LU[c * NEM + pos] = v[c];
+          }
+        if (bad)
           atomicExch(sing, 1);
       }
     else
       {
-        const int t0 = tid - 32, TT = T - 32;
+        const int t0 = tid - 32 * NLW, TT = T - 32 * NLW;
         for (int idx = t0; idx < NEM * (nK + 1); idx += TT)
           {
             const int i = idx % NEM, c = idx / NEM;
             double    x = 0.;
             if (i < nE)
               {
-                if (LEAF)
-                  x = own(e0[i], c < nK ? km[c] : -1);
-                else if (c == nK)
-                  x = kid(0, e0[i], -1) + kid(1, e1[i], -1);
+                if (c == nK)
+                  {
+                    x = rhs(0, erp[i], ers[i], eco[i]);
+                    if (!LEAF)
+                      x += rhs(1, erp[NEM + i], ers[NEM + i], eco[NEM + i]);
+                  }
                 else
                   {
-                    const int s = km[c] >> NDKidBit;
-                    x           = kid(s, s ? e1[i] : e0[i], km[c] & KM);
+                    const int e = kid[c] * NEM + i;
+                    x           = entry(erp[e], ers[e], eco[e], kco[c]);
                   }
               }
             Bs[c * LDW + i] = x;
@@ -381,18 +391,7 @@ namespace ddhdg
         for (int idx = t0; idx < nK * NEM; idx += TT)
           {
             const int r = idx % nK, j = idx / nK;
-            double    x = 0.;
-            if (j < nE)
-              {
-                if (LEAF)
-                  x = own(km[r], e0[j]);
-                else
-                  {
-                    const int s = km[r] >> NDKidBit;
-                    x           = kid(s, km[r] & KM, s ? e1[j] : e0[j]);
-                  }
-              }
-            Ks[r * LDW + j] = -x;
+            Ks[r * LDW + j] = j < nE ? -entry(krp[r], krs[r], kco[r], eco[kid[r] * NEM + j]) : 0.;
           }
       }
     __syncthreads();
@@ -451,36 +450,38 @@ namespace ddhdg
       {
         const int r0 = (tile % rt) * 16, c0 = (tile / rt) * 32;
         double    acc[2][4][2];
-        int       kr[2];
+        {
+          const double *rp[2];
+          double        rs[2];
+          int           rk[2], ro[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-          {
-            const int r = r0 + i * 8 + g;
-            kr[i]       = r < nK ? km[r] : -1;
-          }
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int e = 0; e < 2; ++e)
+          for (int i = 0; i < 2; ++i)
             {
-              const int c  = c0 + j * 8 + 2 * tq + e;
-              const int kc = c < nK ? km[c] : -1;
-#pragma unroll
-              for (int i = 0; i < 2; ++i)
-                {
-                  double x = 0.;
-                  if (kr[i] >= 0 && c <= nK)
-                    {
-                      if (LEAF)
-                        x = own(kr[i], kc);
-                      else if (c == nK)
-                        x = kid(kr[i] >> NDKidBit, kr[i] & KM, -1);
-                      else if ((kc >> NDKidBit) == (kr[i] >> NDKidBit))
-                        x = kid(kr[i] >> NDKidBit, kr[i] & KM, kc & KM);
-                    }
-                  acc[i][j][e] = x;
-                }
+              const int r = min(r0 + i * 8 + g, nK - 1);
+              rp[i]       = krp[r];
+              rs[i]       = krs[r];
+              rk[i]       = kid[r];
+              ro[i]       = kco[r];
             }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              {
+                const int c  = c0 + j * 8 + 2 * tq + e;
+                const int ck = c < nK ? kid[c] : -1, co = c < nK ? kco[c] : 0;
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                  {
+                    double x = 0.;
+                    if (ck == rk[i])
+                      x = entry(rp[i], rs[i], ro[i], co);
+                    else if (c == nK)
+                      x = rhs(rk[i], rp[i], rs[i], ro[i]);
+                    acc[i][j][e] = x;
+                  }
+              }
+        }
 #pragma unroll
         for (int ks = 0; ks < NEM / 4; ++ks)
           {
@@ -572,12 +573,148 @@ namespace ddhdg
   // registers; per column a warp max-reduction, one CTA barrier and, for the
   // fronts whose rows need more than one CTA, one exchange of the C
   // candidates through the distributed shared memory of a cluster of C CTAs.
-  // The kernel is a chain of NDPanel dependent column steps; the candidates'
-  // whole rows travel with their keys, so that a step has a single barrier.
+  // The kernel is a chain of NDPanel dependent column steps, bound by the
+  // instructions and latencies of a step, not by any rate: one barrier per
+  // step (the candidates' rows and reciprocals travel with their keys), and
+  // code that stays in the instruction cache: the eight steps of a group are
+  // unrolled, the groups are a loop (all 32 steps unrolled: 47 us per panel,
+  // instruction fetches; all 32 rolled with a rotating row: 25 us, masking).
+  // After a group the row is rotated by its eight columns, so the current
+  // group is always in the first registers.
   constexpr int NDPanel   = 32;
   constexpr int NDPanelT  = 512;           // threads per CTA at most
   constexpr int NDPanelC  = 8;             // CTAs per cluster at most
   constexpr int NDPanelLd = NDPanel + 4;   // shared row stride (= 4 mod 16)
+  constexpr int NDPanelG  = 8;             // columns per group
+  constexpr int NDPanelN  = NDPanel / NDPanelG;
+
+  template <int CL>
+  struct NDPanelShared
+  {
+    static constexpr int NW = NDPanelT / 32;
+    double   wrow[2][NW][NDPanel]; // candidate row per warp (the columns still active)
+    double   crow[2][CL][NDPanel]; // candidate row per CTA of the cluster
+    // pivot rows by columns: [0] as they are, [1] rows and columns reversed
+    double   LU[2][NDPanel][NDPanel + 2];
+    double   whr[2][NW], chr[2][CL]; // reciprocal pivots
+    double   rd[NDPanel];            // reciprocals of the diagonal of U (1 beyond w)
+    unsigned wkey[2][NW], ckey[2][CL];
+    int      wid[2][NW], cid[2][CL];
+    int      ppos[NDPanel]; // list positions of the pivot rows
+  };
+
+  // one group of NDPanelG column steps, columns j0 .. j0 + 7 in v[0 .. 7];
+  // nact of the blocks of eight columns are still active (this one included)
+  template <int CL>
+  __device__ __forceinline__ void
+  nd_panel_group(double (&v)[NDPanel], NDPanelShared<CL> &S, int j0, int nact, int w, int t, int rank, bool &used,
+                 int &mypos, int *sing)
+  {
+    namespace cg   = cooperative_groups;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int jj = 0; jj < NDPanelG; ++jj)
+      {
+        constexpr int  PK   = 2; // columns per 16-byte access
+        const int      buf  = jj & 1;
+        const double   x0   = v[jj];
+        const unsigned key  = used ? 0u : nd_pivot_key(x0);
+        const double   hx   = (x0 != 0.) ? 1. / x0 : 0.; // overlaps the reduction
+        const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
+        const int      src  = __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1;
+        if (lane == src)
+          {
+            double2 *dst = reinterpret_cast<double2 *>(S.wrow[buf][warp]);
+#pragma unroll
+            for (int k = (jj + 1) / PK * PK; k < NDPanelG; k += PK)
+              dst[k / PK] = make_double2(v[k], v[k + 1]);
+#pragma unroll
+            for (int b = 1; b < NDPanelN; ++b)
+              if (b < nact)
+#pragma unroll
+                for (int k = b * NDPanelG; k < (b + 1) * NDPanelG; k += PK)
+                  dst[k / PK] = make_double2(v[k], v[k + 1]);
+            S.whr[buf][warp]  = hx;
+            S.wkey[buf][warp] = kmax;
+            S.wid[buf][warp]  = t;
+          }
+        __syncthreads();
+        const unsigned k2 = lane < nw ? S.wkey[buf][lane] : 0u;
+        const unsigned m2 = __reduce_max_sync(0xffffffffu, k2);
+        const int      ww = __ffs(__ballot_sync(0xffffffffu, lane < nw && k2 == m2)) - 1;
+        const double  *prow = S.wrow[buf][ww];
+        double         hr   = S.whr[buf][ww];
+        int            pid  = S.wid[buf][ww];
+        if (CL > 1)
+          {
+            cg::cluster_group cl = cg::this_cluster();
+            if (warp < CL)
+              {
+                double *dst = cl.map_shared_rank(&S.crow[buf][rank][0], warp);
+                dst[lane]   = prow[lane]; // the inactive columns are not read
+                if (lane == 0)
+                  {
+                    *cl.map_shared_rank(&S.ckey[buf][rank], warp) = m2;
+                    *cl.map_shared_rank(&S.cid[buf][rank], warp)  = pid;
+                    *cl.map_shared_rank(&S.chr[buf][rank], warp)  = hr;
+                  }
+              }
+            cl.sync();
+            const unsigned k3 = lane < CL ? S.ckey[buf][lane] : 0u;
+            const unsigned m3 = __reduce_max_sync(0xffffffffu, k3);
+            const int      cc = __ffs(__ballot_sync(0xffffffffu, lane < CL && k3 == m3)) - 1;
+            prow              = S.crow[buf][cc];
+            hr                = S.chr[buf][cc];
+            pid               = S.cid[buf][cc];
+          }
+        const bool    me = !used && t == pid;
+        const double  l  = (used || me) ? 0. : -x0 * hr;
+        const double2 *pr = reinterpret_cast<const double2 *>(prow);
+#pragma unroll
+        for (int k = (jj + 1) / PK * PK; k < NDPanelG; k += PK)
+          {
+            const double2 p = pr[k / PK];
+            if (k > jj)
+              v[k] = fma(l, p.x, v[k]);
+            v[k + 1] = fma(l, p.y, v[k + 1]);
+          }
+#pragma unroll
+        for (int b = 1; b < NDPanelN; ++b)
+          if (b < nact)
+#pragma unroll
+            for (int k = b * NDPanelG; k < (b + 1) * NDPanelG; k += PK)
+              {
+                const double2 p = pr[k / PK];
+                v[k]            = fma(l, p.x, v[k]);
+                v[k + 1]        = fma(l, p.y, v[k + 1]);
+              }
+        if (!used && !me)
+          v[jj] = -l;
+        if (me)
+          {
+            used  = true;
+            mypos = j0 + jj;
+            if (!(fabs(x0) > 0.) || !isfinite(x0))
+              atomicExch(sing, 1);
+          }
+        if (threadIdx.x == 0 && j0 + jj < w)
+          {
+            S.ppos[j0 + jj] = pid;
+            S.rd[j0 + jj]   = hr;
+          }
+      }
+    // the finished columns to the end
+    double f[NDPanelG];
+#pragma unroll
+    for (int k = 0; k < NDPanelG; ++k)
+      f[k] = v[k];
+#pragma unroll
+    for (int k = NDPanelG; k < NDPanel; ++k)
+      v[k - NDPanelG] = v[k];
+#pragma unroll
+    for (int k = 0; k < NDPanelG; ++k)
+      v[NDPanel - NDPanelG + k] = f[k];
+  }
 
   template <int CL>
   __global__ void __launch_bounds__(NDPanelT, 1)
@@ -585,22 +722,14 @@ namespace ddhdg
                   double *luf, int32_t *perm, double *tinv, int *sing)
   {
     namespace cg = cooperative_groups;
-    constexpr int       NW = NDPanelT / 32;
-    __shared__ __align__(16) double wrow[2][NW][NDPanel]; // candidate row per warp
-    __shared__ unsigned wkey[2][NW];
-    __shared__ int      wid[2][NW];
-    __shared__ __align__(16) double crow[2][CL][NDPanel]; // candidate row per CTA of the cluster
-    __shared__ unsigned ckey[2][CL];
-    __shared__ int      cid[2][CL];
-    __shared__ double   Ls[NDPanel][NDPanel + 1]; // pivot rows in pivot order
-    __shared__ int      ppos[NDPanel];            // their list positions
-    const NDNode       &n  = nodes[blockIdx.x / CL];
-    const int           nE = n.nE;
+    __shared__ __align__(16) NDPanelShared<CL> S;
+    const NDNode &n  = nodes[blockIdx.x / CL];
+    const int     nE = n.nE;
     if (nE <= k0)
       return; // every CTA of the cluster
     const int rank = CL > 1 ? (int)(blockIdx.x % CL) : 0;
     const int m = nE - k0, w = min(NDPanel, m);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x, nw = T >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
     const int t    = rank * T + tid; // position in the row list
     const bool has = t < m;
     const int  row = has ? (k0 ? ul_in[n.poff + t] : t) : 0;
@@ -611,83 +740,37 @@ namespace ddhdg
       v[c] = (has && c < w) ? A[(int64_t)c * n.ld + row] : 0.;
     bool used  = !has;
     int  mypos = -1;
+    if (rank == 0)
+      for (int i = tid; i < 2 * NDPanel * (NDPanel + 2); i += T)
+        (&S.LU[0][0][0])[i] = 0.;
+    if (tid < NDPanel)
+      S.rd[tid] = 1.;
     if (CL > 1)
       cg::this_cluster().sync(); // every CTA of the cluster runs before its shared memory is written
+    else
+      __syncthreads();
+#pragma unroll 1
+    for (int g = 0; g < NDPanelN; ++g)
+      nd_panel_group<CL>(v, S, g * NDPanelG, NDPanelN - g, w, t, rank, used, mypos, sing);
+    if (mypos >= 0)
+      {
+        double *d0 = &S.LU[0][0][mypos], *d1 = &S.LU[1][NDPanel - 1][NDPanel - 1 - mypos];
+        if (CL > 1)
+          {
+            d0 = cg::this_cluster().map_shared_rank(d0, 0);
+            d1 = cg::this_cluster().map_shared_rank(d1, 0);
+          }
 #pragma unroll
-    for (int j = 0; j < NDPanel; ++j)
-      if (j < w)
-        {
-          const int      buf  = j & 1;
-          const unsigned key  = used ? 0u : nd_pivot_key(v[j]);
-          const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
-          const int      src  = __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1;
-          if (lane == src)
-            {
-#pragma unroll
-              for (int c = 0; c < NDPanel; c += 2)
-                *reinterpret_cast<double2 *>(&wrow[buf][warp][c]) = make_double2(v[c], v[c + 1]);
-              wkey[buf][warp] = kmax;
-              wid[buf][warp]  = t;
-            }
-          __syncthreads();
-          const unsigned k2 = lane < nw ? wkey[buf][lane] : 0u;
-          const unsigned m2 = __reduce_max_sync(0xffffffffu, k2);
-          const int      ww = __ffs(__ballot_sync(0xffffffffu, lane < nw && k2 == m2)) - 1;
-          const double  *prow = wrow[buf][ww];
-          int            pid  = wid[buf][ww];
-          if (CL > 1)
-            {
-              cg::cluster_group cl = cg::this_cluster();
-              if (warp < CL)
-                {
-                  double *dst = cl.map_shared_rank(&crow[buf][rank][0], warp);
-                  dst[lane]   = prow[lane];
-                  if (lane == 0)
-                    {
-                      *cl.map_shared_rank(&ckey[buf][rank], warp) = m2;
-                      *cl.map_shared_rank(&cid[buf][rank], warp)  = pid;
-                    }
-                }
-              cl.sync();
-              const unsigned k3 = lane < CL ? ckey[buf][lane] : 0u;
-              const unsigned m3 = __reduce_max_sync(0xffffffffu, k3);
-              const int      cc = __ffs(__ballot_sync(0xffffffffu, lane < CL && k3 == m3)) - 1;
-              prow              = crow[buf][cc];
-              pid               = cid[buf][cc];
-            }
-          const double d  = prow[j];
-          const double hr = (d != 0.) ? 1. / d : 0.;
-          if (warp == 0)
-            {
-              if (rank == 0)
-                Ls[j][lane] = prow[lane];
-              if (lane == 0)
-                {
-                  ppos[j] = pid;
-                  if (rank == 0 && (!(fabs(d) > 0.) || !isfinite(d)))
-                    atomicExch(sing, 1);
-                }
-            }
-          if (!used)
-            {
-              if (t == pid)
-                {
-                  used  = true;
-                  mypos = j;
-                }
-              else
-                {
-                  const double l = v[j] * hr;
-                  v[j]           = l;
-#pragma unroll
-                  for (int c = j + 1; c < NDPanel; ++c)
-                    v[c] -= l * prow[c];
-                }
-            }
-        }
-    __syncthreads(); // Ls, ppos
-    const int ldl = n.nEp;
-    double   *LUF = luf + n.luoff + (int64_t)k0 * ldl + k0;
+        for (int c = 0; c < NDPanel; ++c)
+          {
+            d0[c * (NDPanel + 2)]  = v[c];
+            d1[-c * (NDPanel + 2)] = v[c];
+          }
+      }
+    if (CL > 1)
+      cg::this_cluster().sync(); // also: no CTA's shared memory is written after this
+    else
+      __syncthreads();
     if (mypos >= 0)
       perm[n.poff + k0 + mypos] = row;
     else if (has)
@@ -695,7 +778,7 @@ namespace ddhdg
         int below = 0;
 #pragma unroll
         for (int j = 0; j < NDPanel; ++j)
-          below += (j < w && ppos[j] < t) ? 1 : 0;
+          below += (j < w && S.ppos[j] < t) ? 1 : 0;
         ul_out[n.poff + t - below] = row;
 #pragma unroll
         for (int c = 0; c < NDPanel; ++c)
@@ -703,51 +786,55 @@ namespace ddhdg
       }
     if (rank == 0)
       {
-        for (int idx = tid; idx < w * w; idx += T)
-          LUF[(int64_t)(idx / w) * ldl + idx % w] = Ls[idx % w][idx / w];
         // inverses of the unit lower and of the upper diagonal block (identity
-        // beyond w), a lane per column
+        // beyond w), a lane per column: substitution by columns, the upper
+        // block on its reversed copy; groups as above
         if (warp < 2)
           {
-            double x[NDPanel];
-            if (warp == 0)
+            const bool up = warp == 1;
+            double     y[NDPanel];
+#pragma unroll
+            for (int r = 0; r < NDPanel; ++r)
+              y[r] = ((up ? NDPanel - 1 - r : r) == lane) ? 1. : 0.;
+            double *out = tinv + n.tioff + ((int64_t)(k0 / NDPanel) * 2 + warp) * NDPanel * NDPanel + lane * NDPanel;
+#pragma unroll 1
+            for (int g = 0; g < NDPanelN; ++g)
               {
 #pragma unroll
-                for (int r = 0; r < NDPanel; ++r)
+                for (int jj = 0; jj < NDPanelG; ++jj)
                   {
-                    double y = (r == lane) ? 1. : 0.;
-                    if (r < w)
+                    const int c = g * NDPanelG + jj;
+                    if (up)
+                      y[jj] *= S.rd[NDPanel - 1 - c];
+                    const double  x = -y[jj];
+                    const double *f = &S.LU[warp][c][g * NDPanelG];
 #pragma unroll
-                      for (int s = 0; s < r; ++s)
-                        y -= Ls[r][s] * x[s]; // x[s] = 0 for s < lane
-                    x[r] = y;
+                    for (int k = jj + 1; k < NDPanelG; ++k)
+                      y[k] = fma(f[k], x, y[k]);
+#pragma unroll
+                    for (int b = 1; b < NDPanelN; ++b)
+                      if (b < NDPanelN - g)
+#pragma unroll
+                        for (int k = b * NDPanelG; k < (b + 1) * NDPanelG; k += 2)
+                          {
+                            const double2 p = *reinterpret_cast<const double2 *>(f + k);
+                            y[k]            = fma(p.x, x, y[k]);
+                            y[k + 1]        = fma(p.y, x, y[k + 1]);
+                          }
                   }
+#pragma unroll
+                for (int k = 0; k < NDPanelG; ++k)
+                  out[up ? NDPanel - 1 - g * NDPanelG - k : g * NDPanelG + k] = y[k];
+#pragma unroll
+                for (int k = NDPanelG; k < NDPanel; ++k)
+                  y[k - NDPanelG] = y[k];
               }
-            else
-              {
-#pragma unroll
-                for (int r = NDPanel - 1; r >= 0; --r)
-                  {
-                    double y = (r == lane) ? 1. : 0.;
-                    if (r < w)
-                      {
-#pragma unroll
-                        for (int s = r + 1; s < NDPanel; ++s)
-                          if (s < w)
-                            y -= Ls[r][s] * x[s]; // x[s] = 0 for s > lane
-                        y /= Ls[r][r];
-                      }
-                    x[r] = y;
-                  }
-              }
-            double *out = tinv + n.tioff + ((int64_t)(k0 / NDPanel) * 2 + warp) * NDPanel * NDPanel;
-#pragma unroll
-            for (int r = 0; r < NDPanel; r += 2)
-              *reinterpret_cast<double2 *>(out + lane * NDPanel + r) = make_double2(x[r], x[r + 1]);
           }
+        const int ldl = n.nEp;
+        double   *LUF = luf + n.luoff + (int64_t)k0 * ldl + k0;
+        for (int idx = tid; idx < w * w; idx += T)
+          LUF[(int64_t)(idx / w) * ldl + idx % w] = S.LU[0][idx / w][idx % w];
       }
-    if (CL > 1)
-      cg::this_cluster().sync(); // no CTA leaves while its shared memory may still be written
   }
 
   __device__ __forceinline__ void
@@ -1118,14 +1205,21 @@ namespace ddhdg
           }
         if (t.j != t.i)
           {
+            // all fragments of the block first: the loads overlap
+            double a[NDPanel / 4], b[NDPanel / 4][2];
 #pragma unroll
             for (int ks = 0; ks < NDPanel / 4; ++ks)
               {
-                const double a = -A[(ks * 4 + q) * NDPanelLd + mt * 8 + g];
+                a[ks] = -A[(ks * 4 + q) * NDPanelLd + mt * 8 + g];
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
-                  dmma8x8x4(acc[j][0], acc[j][1], a, Bs[((nt + j) * 8 + g) * ldb + t.j * NDPanel + ks * 4 + q]);
+                  b[ks][j] = Bs[((nt + j) * 8 + g) * ldb + t.j * NDPanel + ks * 4 + q];
               }
+#pragma unroll
+            for (int ks = 0; ks < NDPanel / 4; ++ks)
+#pragma unroll
+              for (int j = 0; j < 2; ++j)
+                dmma8x8x4(acc[j][0], acc[j][1], a[ks], b[ks][j]);
           }
         else
           {
@@ -1233,43 +1327,54 @@ namespace ddhdg
     for (int s = 0; s < NDGStages - 1; ++s)
       issue(s, s);
     double acc[4][4][2];
-    if (SCHUR)
+    if (SCHUR && n.cell >= 0)
       {
-        const NDFront  F_{n, Cc, maps + n.map, fronts};
+        const NDFront F_{n, Cc, maps + n.map, fronts};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            {
+              const int c = n0 + wn + j * 8 + 2 * q + e;
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                {
+                  const int r  = m0 + wm + i * 8 + g;
+                  acc[i][j][e] = (r < m && c < nn) ? F_.KK(r, c) : 0.;
+                }
+            }
+      }
+    else if (SCHUR)
+      {
+        // rows as pointers into the child that holds them, columns as offsets
         const int32_t *km = maps + n.map + 2 * n.nE;
         constexpr int  KM = (1 << NDKidBit) - 1;
-        int            kr[4];
+        const double  *rp[4];
+        int            rk[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           {
-            const int r = m0 + wm + i * 8 + g;
-            kr[i]       = (n.cell < 0 && r < m) ? km[r] : -1;
+            const int k = km[min(m0 + wm + i * 8 + g, m - 1)];
+            rk[i]       = k >> NDKidBit;
+            rp[i]       = fronts + (rk[i] ? n.coff[1] : n.coff[0]) + (rk[i] ? n.cEp[1] : n.cEp[0]) + (k & KM);
           }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
           for (int e = 0; e < 2; ++e)
             {
-              const int c  = n0 + wn + j * 8 + 2 * q + e;
-              const int kc = (n.cell < 0 && c < n.nK) ? km[c] : -1;
+              const int     c  = n0 + wn + j * 8 + 2 * q + e;
+              const int     k  = km[min(c, n.nK - 1)];
+              const int     ck = c < n.nK ? k >> NDKidBit : -1;
+              const int64_t co = (int64_t)(k & KM) * (ck > 0 ? n.cld[1] : n.cld[0]);
 #pragma unroll
               for (int i = 0; i < 4; ++i)
                 {
-                  const int r = m0 + wm + i * 8 + g;
-                  double    x = 0.;
-                  if (r < m && c < nn)
-                    {
-                      if (n.cell >= 0)
-                        x = F_.KK(r, c);
-                      else
-                        {
-                          const int s = kr[i] >> NDKidBit;
-                          if (c == n.nK)
-                            x = nd_kid(n, fronts, s, kr[i] & KM, s ? n.cnK[1] : n.cnK[0]);
-                          else if ((kc >> NDKidBit) == s)
-                            x = nd_kid(n, fronts, s, kr[i] & KM, kc & KM);
-                        }
-                    }
+                  double x = 0.;
+                  if (ck == rk[i])
+                    x = rp[i][co];
+                  else if (c == n.nK)
+                    x = rp[i][(int64_t)(rk[i] ? n.cnK[1] : n.cnK[0]) * (rk[i] ? n.cld[1] : n.cld[0])];
                   acc[i][j][e] = x;
                 }
             }

@@ -36,9 +36,9 @@ namespace ddhdg
     constexpr int    SolveRows  = 576; // rows of B that stay in shared memory (32 columns, 185 KB with the stages)
 
     Class
-    class_of(int nE, int nK, int Nt)
+    class_of(int nE, int nK)
     {
-      if (nE <= NDSmallE && nd_small_smem(nd_small_class(nE), nK, Nt) <= SmallSmem)
+      if (nE <= NDSmallE && nd_small_smem(nd_small_class(nE), nK) <= SmallSmem)
         return nE <= 4 ? Small4 : nE <= 12 ? Small12 : nE <= 20 ? Small20 : nE <= 28 ? Small28 : Small36;
       return nE <= PanelRows ? Panels : Library;
     }
@@ -221,7 +221,6 @@ namespace ddhdg
         return bad(err, "unsupported mesh for the nested-dissection solve");
       if (M.nfaces * (int64_t)M.nd > INT32_MAX)
         return bad(err, "too many trace dofs for 32-bit dof lists");
-      const int Nt = M.F * M.nd;
       cell_faces.assign(M.ncells * M.F, 0);
       for (int64_t c = 0; c < M.ncells; ++c)
         for (int f = 0; f < M.F; ++f)
@@ -238,7 +237,7 @@ namespace ddhdg
           HostNode &h = tree[i];
           if (h.nE == 0)
             continue;
-          cls[i] = class_of(h.nE, h.nK, Nt);
+          cls[i] = class_of(h.nE, h.nK);
           h.doff = doff;
           doff += h.nE + h.nK;
           ids.push_back(i);
@@ -334,7 +333,7 @@ namespace ddhdg
                   n.cEp[s]  = (int)even(c.nE);
                   n.cld[s]  = n.cEp[s] + (int)even(c.nK);
                 }
-              if (n.ccell[s] >= 0 && class_of(h.nE, h.nK, Nt) >= Panels)
+              if (n.ccell[s] >= 0 && class_of(h.nE, h.nK) >= Panels)
                 return bad(err, "nested dissection: a large front over an interior cell");
             }
           const std::array<int, 4> key{
@@ -678,9 +677,10 @@ namespace ddhdg
     launch_small(const Batch &b, const NDNode *nodes, const int32_t *maps, const NDCells &C, int *sing, double *fronts,
                  cudaStream_t s)
     {
-      const size_t smem = nd_small_smem(NEM, b.maxK, C.Nt);
-      // warp 0 factorises, the others stage; a thread per column solves for W
-      const int T = b.maxK + 1 > 128 ? 256 : 128;
+      const size_t smem = nd_small_smem(NEM, b.maxK);
+      // one or two warps factorise, the others stage; a thread per column
+      // solves for W; 16 warps where one CTA fills the SM's shared memory
+      const int T = NEM > 28 && smem > 110 * 1024 ? 512 : b.maxK + 1 > 128 ? 256 : 128;
       if (b.leaf)
         nd_small_kernel<NEM, true><<<b.count, T, smem, s>>>(nodes, maps, C, b.maxK, sing, fronts);
       else
