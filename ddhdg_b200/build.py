@@ -8,8 +8,9 @@ import tempfile
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libddhdg_b200.so")
-# compiled side by side, one object per source
-SOURCES = ["hdg_capi.cu", "hdg_ndsolve.cu"]
+# translation units, compiled side by side: (source, extra flags)
+UNITS = [("hdg_capi.cu", []), ("hdg_ndsolve.cu", [])] + \
+    [(s, [f"-DDDHDG_DIM={d}"]) for s in ("hdg_condense_dim.cu", "hdg_batch_dim.cu") for d in (2, 3, 1)]
 HEADER = os.path.join(HERE, "..", "include", "ddhdg_b200.h")
 
 NVCC_FLAGS = [
@@ -37,9 +38,9 @@ def build(force=False, verbose=False):
         return LIB
     with tempfile.TemporaryDirectory() as tmp:
         objs, jobs = [], []
-        for s in SOURCES:
-            objs.append(os.path.join(tmp, s + ".o"))
-            cmd = [nvcc()] + NVCC_FLAGS + ["-c", "-o", objs[-1], os.path.join(CSRC, s)]
+        for i, (s, extra) in enumerate(UNITS):
+            objs.append(os.path.join(tmp, f"{i}_{s}.o"))
+            cmd = [nvcc()] + NVCC_FLAGS + extra + ["-c", "-o", objs[-1], os.path.join(CSRC, s)]
             if verbose:
                 print(" ".join(cmd), file=sys.stderr)
             jobs.append((cmd, subprocess.Popen(cmd)))

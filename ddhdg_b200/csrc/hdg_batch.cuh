@@ -5,7 +5,7 @@
 // The reference assembles one device at a time, its per-cell worker run over
 // the cells by WorkStream (include/assembling_methods.template.h:67-88).
 // Here a work list of tiles (device, range of its cells) is consumed by one
-// grid of CTAs of BatchTPB threads: every CTA takes the next tile from a
+// grid of CTAs of batch_threads threads: every CTA takes the next tile from a
 // counter, loads that device's launch parameters into shared memory and runs
 // the per-degree body on the tile's cells (the unit-cell constant tables of
 // every degree travel in the constant bank): two warps on two cells at a time
@@ -27,8 +27,20 @@
 
 namespace ddhdg
 {
-  constexpr int BatchTPB  = 64;          // 2 warps: two cells at a time, or one CTA-per-cell cell
-  constexpr int BatchWarp = BatchTPB / 32;
+  // threads per CTA by dimension: a cell per warp at a time, or one
+  // CTA-per-cell cell.  Two warps; three in 3D, whose degree-2 cells factorise
+  // a row per thread (81 rows) and whose degree-1 cells share an SM in sixes
+  // either way.
+  __host__ __device__ constexpr int
+  batch_threads(int dim)
+  {
+    return dim == 3 ? 96 : 64;
+  }
+  __host__ __device__ constexpr int
+  batch_warps(int dim)
+  {
+    return batch_threads(dim) / 32;
+  }
   constexpr int BatchRTPB = 256;         // reconstruction: 8 warps
 
   struct BatchJob
@@ -105,15 +117,15 @@ namespace ddhdg
         // the device's face-flux table of the tt epilogue, after the warps'
         // workspaces (as the single-device kernel stages it)
         constexpr int NR  = CTab<DIM, K>::Fq * CTab<DIM, K>::Ft;
-        double       *rqr = smem + BatchWarp * wo.total;
-        for (int i = threadIdx.x; i < NR; i += BatchTPB)
+        double       *rqr = smem + batch_warps(DIM) * wo.total;
+        for (int i = threadIdx.x; i < NR; i += batch_threads(DIM))
           rqr[i] = P.tables[P.to.RQr + i];
         __syncthreads();
         condense3_cells<DIM, K, JT>(P, batch_tab<K>(C), smem + warp * wo.total, piv[warp], t.begin + warp,
-                                    t.end, BatchWarp, rqr);
+                                    t.end, batch_warps(DIM), rqr);
       }
     else if constexpr (sizeof(JT) == 8)
-      condense2_cells<DIM, K, BatchTPB>(P, smem, blockIdx.x, t.begin, t.end, 1);
+      condense2_cells<DIM, K, batch_threads(DIM)>(P, smem, blockIdx.x, t.begin, t.end, 1);
   }
 
   // The precisions a batch holds: FP64 devices only, mixed-precision
@@ -123,7 +135,7 @@ namespace ddhdg
   // registers), the occupancy of the single-device mixed kernel; the others
   // for four (the FP64 bodies take 255 registers, and the mixed bodies
   // beside them add spills).  Small CTAs keep several CTA-per-cell cells
-  // on an SM, so that their serial LU panels overlap.
+  // on an SM, so that their serial pivot steps overlap.
   enum BatchPrec : int
   {
     BatchFP64  = 0,
@@ -133,12 +145,12 @@ namespace ddhdg
 
   // counter: tiles handed out so far (zero at launch)
   template <int DIM, int PREC>
-  __global__ void __launch_bounds__(BatchTPB, PREC == BatchMixed ? 8 : 4)
+  __global__ void __launch_bounds__(batch_threads(DIM), DIM == 3 ? (PREC == BatchMixed ? 5 : 2) : (PREC == BatchMixed ? 8 : 4))
   batch_condense_kernel(const BatchJob *__restrict__ jobs, const BatchTile *__restrict__ tiles,
                         int ntiles, int *counter, const __grid_constant__ BatchTabs<DIM> C)
   {
     extern __shared__ __align__(16) double smem[];
-    __shared__ int                   piv[BatchWarp][32];
+    __shared__ int                   piv[batch_warps(DIM)][32];
     __shared__ __align__(16) KParams Ps;
     __shared__ int                   s_tile, s_k;
     for (;;)

@@ -25,6 +25,7 @@
 #include "hdg_condense.cuh"
 #include "hdg_condense3.cuh"
 #include "hdg_kernels.cuh"
+#include "hdg_launch.h"
 #include "hdg_ndsolve.h"
 #include "hdg_plain.cuh"
 #include "hdg_tables.h"
@@ -496,113 +497,51 @@ namespace
     return P;
   }
 
-  using ReconstructFn = void (*)(KParams, const double *, double *);
-
-  // one condense kernel of a (dim, degree): its address (attributes,
-  // occupancy) and a launcher that builds its parameters
-  struct CondenseKernel
-  {
-    const void *fn = nullptr;
-    void (*launch)(const Tables &, const KParams &, int, int, size_t, cudaStream_t) = nullptr;
-  };
-
-  template <int D, int K>
-  void
-  fill_ctab(const Tables &T, CTab<D, K> &C)
-  {
-    auto put = [](double *dst, size_t n, const std::vector<double> &src) {
-      std::memcpy(dst, src.data(), std::min(n, src.size()) * sizeof(double));
-    };
-    put(C.phi_c, sizeof(C.phi_c) / sizeof(double), T.phi_c);
-    put(C.RTk, sizeof(C.RTk) / sizeof(double), T.RTk);
-    put(C.phi_f, sizeof(C.phi_f) / sizeof(double), T.phi_f);
-    put(C.RTr, sizeof(C.RTr) / sizeof(double), T.RTr);
-    put(C.RQk, sizeof(C.RQk) / sizeof(double), T.RQk);
-    put(C.RQr, sizeof(C.RQr) / sizeof(double), T.RQr);
-    put(C.xi, sizeof(C.xi) / sizeof(double), T.xi);
-  }
-
-  template <int D, int K, typename JT>
-  void
-  launch_condense(const Tables &T, const KParams &P, int grid, int threads, size_t smem,
-                  cudaStream_t s)
-  {
-    if constexpr (3 * Dims<D, K>::nb <= 32)
-      {
-        CTab<D, K> C;
-        fill_ctab(T, C);
-        condense3_kernel<D, K, JT><<<grid, threads, smem, s>>>(P, C);
-      }
-    else
-      condense2_kernel<D, K><<<grid, threads, smem, s>>>(P);
-  }
-
-  // mixed: the FP32-Jacobian variant of the warp-per-cell kernel; false when
-  // the (dim, degree) has none (the caller rejects mixed precision there)
-  template <int D, int K>
-  bool
-  pick(CondenseKernel &cf, ReconstructFn &rf, bool mixed)
-  {
-    // warp-per-cell register kernel when one lane can own one row of the
-    // scalar system, CTA-per-cell shared-memory kernel otherwise
-    rf = reconstruct_kernel<D, K>;
-    if constexpr (3 * Dims<D, K>::nb <= 32)
-      {
-        if (mixed)
-          {
-            cf.fn     = reinterpret_cast<const void *>(condense3_kernel<D, K, float>);
-            cf.launch = launch_condense<D, K, float>;
-          }
-        else
-          {
-            cf.fn     = reinterpret_cast<const void *>(condense3_kernel<D, K, double>);
-            cf.launch = launch_condense<D, K, double>;
-          }
-        return true;
-      }
-    else
-      {
-        cf.fn     = reinterpret_cast<const void *>(condense2_kernel<D, K>);
-        cf.launch = launch_condense<D, K, double>;
-        return !mixed;
-      }
-  }
-
   bool
   kernels_for(int dim, int k, CondenseKernel &cf, ReconstructFn &rf, bool mixed = false)
   {
-    switch (dim * 10 + k)
+    switch (dim)
       {
-        case 11: return pick<1, 1>(cf, rf, mixed);
-        case 12: return pick<1, 2>(cf, rf, mixed);
-        case 13: return pick<1, 3>(cf, rf, mixed);
-        case 21: return pick<2, 1>(cf, rf, mixed);
-        case 22: return pick<2, 2>(cf, rf, mixed);
-        case 23: return pick<2, 3>(cf, rf, mixed);
-        case 31: return pick<3, 1>(cf, rf, mixed);
-        case 32: return pick<3, 2>(cf, rf, mixed);
+        case 1: return condense_kernels<1>(k, cf, rf, mixed);
+        case 2: return condense_kernels<2>(k, cf, rf, mixed);
+        case 3: return condense_kernels<3>(k, cf, rf, mixed);
         default: return false;
       }
   }
 
-  // table staging and placement of the right-hand-side block R so that one
-  // cell's workspace (one CTA of CondenseTPB threads) fits in the 227 KB of
-  // shared memory of a CTA; R moves to global memory only when nothing else
-  // makes it fit
+  // Warps (cells) per CTA of the register kernel: as many as its launch bound
+  // and shared memory allow (mixed: two CTAs per SM), but no more than spread
+  // the cells over every SM (a small device is bound by one cell's latency,
+  // which grows with the warps sharing an SM).
   int
-  launch_shape(const ddhdg_ctx *c, const Mode &m, int &stage, bool &r_global, size_t &smem)
+  condense3_wpb(const ddhdg_ctx *c, size_t per, int64_t cells, bool mixed)
+  {
+    // 227 KB per CTA, less the kernel's static arrays (face-flux table, pivots)
+    const int     wmax = condense3_max_warps(c->nb, mixed ? 4 : 8);
+    const int64_t stat = (int64_t)c->F * c->nqf * c->F * c->nf * 8 + wmax * 3 * c->nb * 4 + 64;
+    const int64_t most = std::min<int64_t>(wmax, (mixed ? 110 * 1024 : 227 * 1024 - stat) / (int64_t)per);
+    const int64_t spread = std::max<int64_t>(1, (cells + c->sm_count - 1) / c->sm_count);
+    return (int)std::min(most, spread);
+  }
+
+  // placement of the right-hand-side block R so that one cell's workspace
+  // (one CTA) fits in the 227 KB of shared memory of a CTA; R moves to global
+  // memory only when nothing else makes it fit.  The tables are read through
+  // L1: staged, they take the room of a second pair of cells (2D k = 3:
+  // 4.92 ms with 128 threads and staged tables, 4.35 ms with 64 and four cells
+  // per SM, 101 x 101 cells).
+  int
+  launch_shape(const ddhdg_ctx *c, const Mode &m, bool &r_global, size_t &smem)
   {
     const size_t limit = 220 * 1024;
-    const size_t tb    = (((size_t)c->to.total + 1) & ~(size_t)1) * sizeof(double);
     for (int rg = 0; rg < 2; ++rg)
-      for (stage = 1; stage >= 0; --stage)
-        {
-          r_global       = rg != 0;
-          const Ws2Off w = ws2_layout(c->dim, c->nb, c->nf, m.ncomp, m.ncol, r_global);
-          smem           = (stage ? tb : 0) + (size_t)w.total * sizeof(double);
-          if (smem <= limit)
-            return DDHDG_OK;
-        }
+      {
+        r_global       = rg != 0;
+        const Ws2Off w = ws2_layout(c->dim, c->nb, c->nf, m.ncomp, m.ncol, r_global);
+        smem           = (size_t)w.total * sizeof(double);
+        if (smem <= limit)
+          return DDHDG_OK;
+      }
     return fail(DDHDG_BAD_ARG, "the per-cell workspace does not fit in shared memory");
   }
 
@@ -1234,11 +1173,11 @@ condense_range(ddhdg_ctx *c, const double *cell_state, const double *trace_state
   int64_t units;
   if (3 * c->nb <= 32)
     {
-      // warp per cell: as many warps per CTA as shared memory allows
+      // as many cells per CTA as shared memory allows
       // mixed: two CTAs per SM (the FP32 kernel is built for 128 registers)
       const Ws3Off w   = ws3_layout(c->dim, c->nb, c->nf, m.ncomp, m.ncol, mixed ? 4 : 8);
       const size_t per = (size_t)w.total * sizeof(double);
-      int          wpb = (int)std::min<size_t>(Condense3MaxWPB, (mixed ? 110 : 220) * 1024 / per);
+      int          wpb = condense3_wpb(c, per, c1 - c0, mixed);
       if (wpb < 1)
         return fail(DDHDG_BAD_ARG, "the per-cell workspace does not fit in shared memory");
       P.wpb   = wpb;
@@ -1249,13 +1188,11 @@ condense_range(ddhdg_ctx *c, const double *cell_state, const double *trace_state
     }
   else
     {
-      int  stage;
       bool r_global;
-      if ((r = launch_shape(c, m, stage, r_global, smem)))
+      if ((r = launch_shape(c, m, r_global, smem)))
         return r;
       P.wpb   = 1;
-      P.stage = stage;
-      threads = CondenseTPB;
+      threads = condense2_threads(c->nb);
       units   = c1 - c0;
       if (r_global)
         {
@@ -1871,7 +1808,7 @@ ddhdg_assemble_condense_noalloc(ddhdg_ctx *c, const double *cell_state,
     {
       const Ws3Off w   = ws3_layout(c->dim, c->nb, c->nf, m.ncomp, m.ncol, mixed ? 4 : 8);
       const size_t per = (size_t)w.total * sizeof(double);
-      int          wpb = (int)std::min<size_t>(Condense3MaxWPB, (mixed ? 110 : 220) * 1024 / per);
+      int          wpb = condense3_wpb(c, per, c->ncells, mixed);
       if (wpb < 1)
         return fail(DDHDG_BAD_ARG, "the per-cell workspace does not fit in shared memory");
       P.wpb   = wpb;
@@ -1882,12 +1819,10 @@ ddhdg_assemble_condense_noalloc(ddhdg_ctx *c, const double *cell_state,
     }
   else
     {
-      int stage;
-      if ((r = launch_shape(c, m, stage, r_global, smem)))
+      if ((r = launch_shape(c, m, r_global, smem)))
         return r;
       P.wpb   = 1;
-      P.stage = stage;
-      threads = CondenseTPB;
+      threads = condense2_threads(c->nb);
       units   = c->ncells;
     }
   CK(allow_full_dynamic_smem(cf.fn));
@@ -2278,50 +2213,19 @@ struct ddhdg_batch
 
 namespace
 {
-  template <int D>
-  const void *
-  batch_condense_fn_d(int prec)
-  {
-    switch (prec)
-      {
-        case BatchFP64: return reinterpret_cast<const void *>(batch_condense_kernel<D, BatchFP64>);
-        case BatchMixed: return reinterpret_cast<const void *>(batch_condense_kernel<D, BatchMixed>);
-        default: return reinterpret_cast<const void *>(batch_condense_kernel<D, BatchBoth>);
-      }
-  }
   const void *
   batch_condense_fn(int dim, int prec)
   {
-    switch (dim)
-      {
-        case 1: return batch_condense_fn_d<1>(prec);
-        case 2: return batch_condense_fn_d<2>(prec);
-        default: return batch_condense_fn_d<3>(prec);
-      }
+    return dim == 1 ? BatchKernels<1>::condense_fn(prec) :
+           dim == 2 ? BatchKernels<2>::condense_fn(prec) :
+                      BatchKernels<3>::condense_fn(prec);
   }
   const void *
   batch_reconstruct_fn(int dim)
   {
-    switch (dim)
-      {
-        case 1: return reinterpret_cast<const void *>(batch_reconstruct_kernel<1>);
-        case 2: return reinterpret_cast<const void *>(batch_reconstruct_kernel<2>);
-        default: return reinterpret_cast<const void *>(batch_reconstruct_kernel<3>);
-      }
-  }
-
-  // the unit-cell constant tables of every warp-per-cell degree of DIM
-  template <int D>
-  void
-  fill_batch_tabs(BatchTabs<D> &C)
-  {
-    const double unit[3] = {1., 1., 1.};
-    if constexpr (batch_warp<D, 1>)
-      fill_ctab(build_tables(D, 1, unit), C.t1);
-    if constexpr (batch_warp<D, 2>)
-      fill_ctab(build_tables(D, 2, unit), C.t2);
-    if constexpr (batch_warp<D, 3>)
-      fill_ctab(build_tables(D, 3, unit), C.t3);
+    return dim == 1 ? BatchKernels<1>::reconstruct_fn() :
+           dim == 2 ? BatchKernels<2>::reconstruct_fn() :
+                      BatchKernels<3>::reconstruct_fn();
   }
 
   // work lists and launch shapes for the current tile sizes
@@ -2378,7 +2282,7 @@ namespace
     b->ntiles_c     = (int)tc.size();
     b->ntiles_r     = (int)tr.size();
     int per_sm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fc, BatchTPB, b->smem_c));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fc, batch_threads(b->dim), b->smem_c));
     if (per_sm < 1)
       return fail(DDHDG_BAD_ARG, "batched condense kernel does not fit on an SM");
     b->occ_c  = per_sm;
@@ -2400,33 +2304,16 @@ namespace
     return DDHDG_OK;
   }
 
-  template <int D>
-  void
-  batch_launch_condense_d(ddhdg_batch *b, const BatchJob *jobs, const BatchTile *tiles, cudaStream_t s)
-  {
-    static BatchTabs<D>   C; // filled once; the tables do not depend on the device
-    static std::once_flag once;
-    std::call_once(once, [] { fill_batch_tabs<D>(C); });
-    if (b->prec == BatchFP64)
-      batch_condense_kernel<D, BatchFP64><<<b->grid_c, BatchTPB, b->smem_c, s>>>(jobs, tiles, b->ntiles_c, b->counter.p, C);
-    else if (b->prec == BatchMixed)
-      batch_condense_kernel<D, BatchMixed><<<b->grid_c, BatchTPB, b->smem_c, s>>>(jobs, tiles, b->ntiles_c, b->counter.p, C);
-    else
-      batch_condense_kernel<D, BatchBoth><<<b->grid_c, BatchTPB, b->smem_c, s>>>(jobs, tiles, b->ntiles_c, b->counter.p, C);
-  }
-
   int
   batch_launch_condense(ddhdg_batch *b, cudaStream_t s)
   {
     CK(cudaMemsetAsync(b->counter.p, 0, sizeof(int), s));
     const BatchJob  *jobs  = reinterpret_cast<const BatchJob *>(b->d_jobs.p);
     const BatchTile *tiles = reinterpret_cast<const BatchTile *>(b->d_tiles_c.p);
-    switch (b->dim)
-      {
-        case 1: batch_launch_condense_d<1>(b, jobs, tiles, s); break;
-        case 2: batch_launch_condense_d<2>(b, jobs, tiles, s); break;
-        default: batch_launch_condense_d<3>(b, jobs, tiles, s); break;
-      }
+    const auto launch = b->dim == 1 ? BatchKernels<1>::condense :
+                        b->dim == 2 ? BatchKernels<2>::condense :
+                                      BatchKernels<3>::condense;
+    launch(b->prec, b->grid_c, b->smem_c, jobs, tiles, b->ntiles_c, b->counter.p, s);
     CK(cudaGetLastError());
     return DDHDG_OK;
   }
@@ -2438,18 +2325,10 @@ namespace
     const BatchJob  *jobs  = reinterpret_cast<const BatchJob *>(b->d_jobs.p);
     const BatchTile *tiles = reinterpret_cast<const BatchTile *>(b->d_tiles_r.p);
     int             *cnt   = b->counter.p + 1;
-    switch (b->dim)
-      {
-        case 1:
-          batch_reconstruct_kernel<1><<<b->grid_r, BatchRTPB, b->smem_r, s>>>(jobs, tiles, b->ntiles_r, cnt);
-          break;
-        case 2:
-          batch_reconstruct_kernel<2><<<b->grid_r, BatchRTPB, b->smem_r, s>>>(jobs, tiles, b->ntiles_r, cnt);
-          break;
-        default:
-          batch_reconstruct_kernel<3><<<b->grid_r, BatchRTPB, b->smem_r, s>>>(jobs, tiles, b->ntiles_r, cnt);
-          break;
-      }
+    const auto launch = b->dim == 1 ? BatchKernels<1>::reconstruct :
+                        b->dim == 2 ? BatchKernels<2>::reconstruct :
+                                      BatchKernels<3>::reconstruct;
+    launch(b->grid_r, b->smem_r, jobs, tiles, b->ntiles_r, cnt, s);
     CK(cudaGetLastError());
     return DDHDG_OK;
   }
@@ -2572,7 +2451,7 @@ ddhdg_batch_create(const ddhdg_batch_item *items, int n, int thermo, ddhdg_batch
         {
           const Ws3Off w = ws3_layout(c->dim, c->nb, c->nf, m.ncomp, m.ncol, J.mixed ? 4 : 8);
           // the warps' workspaces and the staged face-flux table
-          b->smem_c = std::max(b->smem_c, ((size_t)BatchWarp * w.total +
+          b->smem_c = std::max(b->smem_c, ((size_t)batch_warps(c->dim) * w.total +
                                            (size_t)(c->F * c->nqf) * (c->F * c->nf)) * sizeof(double));
           J.P.wpb        = 1;
           J.P.stage      = 0;

@@ -1,6 +1,6 @@
 // Per-cell assembly + static condensation kernel (sm_100a, FP64).
 //
-// One CTA of CondenseTPB threads works on one cell at a time (persistent grid,
+// One CTA works on one cell at a time (persistent grid,
 // stride loop over cells).  The reference's local system
 // (include/assembling_methods.template.h:269-2160) is restated in block form:
 // the flux unknowns (E, Wn, Wp) are eliminated through the constant mass
@@ -26,10 +26,18 @@
 #include <cuda_runtime.h>
 
 #include "hdg_kernels.cuh"
+#include "hdg_mma.cuh"
 
 namespace ddhdg
 {
-  constexpr int CondenseTPB = 128;
+  // Threads per CTA (cell) by the nodes of a cell: two warps where four cells
+  // share an SM (2D k = 3), eight where one cell fills its shared memory
+  // (3D k = 2).
+  __host__ __device__ constexpr int
+  condense2_threads(int nb)
+  {
+    return nb > 16 ? 256 : 64;
+  }
 
   struct Ws2Off
   {
@@ -78,23 +86,13 @@ namespace ddhdg
     o.r0    = take(3 * nqc);
     o.r1    = take(3 * nqc * dim);
     o.rf    = take(3 * Fq);
-    o.S     = take(Ns * (Ns + 1));
+    o.S     = take(Ns * (Ns + 1)); // rows, then the factors by columns
     o.R     = r_global ? 0 : take(Ns * ncol); // else a slice of KParams::rscratch
     o.g     = take(Nt);
     o.dfl   = take(Nt);
     o.rhsA  = take(Nt);
     o.total = p;
     return o;
-  }
-
-  // D += A B for one 8x8x4 FP64 tile on the tensor path (mma.sync m8n8k4):
-  // lane l holds A[l/4][l%4], B[l%4][l/4] and D[l/4][2(l%4) + {0,1}]
-  __device__ __forceinline__ void
-  cta_dmma8x8x4(double &d0, double &d1, double a, double b)
-  {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
   }
 
   constexpr int CtaLuNB = 8; // panel width of the blocked LU
@@ -124,7 +122,7 @@ namespace ddhdg
   // rounded up)
   template <int T, int NSMAX>
   __device__ void
-  cta_lu_solve(double *S, int ldS, double *R, int ncol, int Ns, int *sh_p, int &sh_sing)
+  cta_lu_blocked(double *S, int ldS, double *R, int ncol, int Ns, int *sh_p, int &sh_sing)
   {
     constexpr int PR = (NSMAX + 31) / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -298,7 +296,7 @@ namespace ddhdg
                     double       b = 0.;
                     if (k < w && vb < nSr + ncol)
                       b = (vb < nSr) ? S[(j0 + k) * ldS + r0 + vb] : R[(j0 + k) * ncol + vb - nSr];
-                    cta_dmma8x8x4(d0, d1, a, b);
+                    dmma8x8x4(d0, d1, a, b);
                   }
                 if (row < Ns)
                   {
@@ -357,7 +355,7 @@ namespace ddhdg
                     const int    k = ks + q;
                     const double a = (k < w && row < j0) ? S[row * ldS + j0 + k] : 0.;
                     const double b = (k < w && cb < ncol) ? R[(j0 + k) * ncol + cb] : 0.;
-                    cta_dmma8x8x4(d0, d1, a, b);
+                    dmma8x8x4(d0, d1, a, b);
                   }
                 if (row < j0)
                   {
@@ -375,12 +373,227 @@ namespace ddhdg
       }
   }
 
+  // The solve of the CTA-per-cell condensation: LU with partial pivoting of
+  // the row-equilibrated S (Ns x Ns, row stride Ns + 1), then Y = S^-1 R in
+  // place of R (Ns x ncol, row stride ncol).
+  // - LU: a row per thread of the first NSMAX / 32 warps, in registers, the
+  //   current column first (rotated by one register per step, so that the
+  //   step loop stays in the instruction cache).  Rows never move: a step
+  //   publishes its warps' candidates (row, reciprocal pivot, key) and has one
+  //   barrier of those warps.  The pivot is within 2^-20 of the largest
+  //   candidate (32-bit keys), ties go to the first row.
+  // - The factors replace S by columns, in pivot order; Y a thread per column
+  //   of R, its entries in registers, groups of eight steps with the factors
+  //   broadcast from shared memory; no barrier.
+  // The chain of Ns pivot steps bounds it; the CTAs sharing an SM overlap.
+  // (A blocked LU with panels in one warp, row swaps and tensor-path trailing
+  // updates had five barriers per eight columns and took half of the kernel.)
+  // Sets sh_sing when a pivot is zero or not finite.
+  template <int T, int NSMAX>
+  __device__ __forceinline__ void
+  cta_lu_solve(double *S, double *R, int ncol, int Ns, int &sh_sing)
+  {
+    constexpr int NW1 = (NSMAX + 31) / 32;          // warps of the LU
+    constexpr int NP  = (NSMAX + 7) / 8 * 8;        // registers of a column of R
+    constexpr int NV  = (NSMAX + 1) / 2 * 2;        // registers of a row
+    static_assert(T >= 32 * NW1, "a thread per row");
+    __shared__ __align__(16) double prow_s[2][NW1][NV];
+    __shared__ double   phr_s[2][NW1], dinv[NSMAX];
+    __shared__ unsigned pkey_s[2][NW1];
+    __shared__ int      pid_s[2][NW1], perm[NSMAX];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ldc = (Ns + 1) & ~1; // column stride of the factors: Ns ldc <= Ns (Ns + 1)
+    if (warp < NW1)
+      {
+        const bool has = tid < Ns;
+        double     v[NV];
+#pragma unroll
+        for (int c = 0; c < NV; ++c)
+          v[c] = (has && c < Ns) ? S[tid * (Ns + 1) + c] : 0.;
+        bool used = !has;
+        int  pos  = -1;
+#pragma unroll 1
+        for (int j = 0; j < NV; ++j)
+          {
+            const double x0 = v[0];
+            if (j >= Ns)
+              {
+                // beyond the system: only the rotation is left
+#pragma unroll
+                for (int k = 1; k < NV; ++k)
+                  v[k - 1] = v[k];
+                v[NV - 1] = x0;
+                continue;
+              }
+            const int      buf  = j & 1;
+            const unsigned key  = used ? 0u : (unsigned)((unsigned long long)__double_as_longlong(fabs(x0)) >> 32) + 1u;
+            const double   hx   = (x0 != 0.) ? 1. / x0 : 0.; // overlaps the reduction
+            const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
+            const int      src  = __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1;
+            if (lane == src)
+              {
+                // finished columns, at the end, are published as zeros
+                double2 *dst = reinterpret_cast<double2 *>(prow_s[buf][warp]);
+#pragma unroll
+                for (int k = 0; k < NV; k += 2)
+                  dst[k / 2] = make_double2(k < NV - j ? v[k] : 0., k + 1 < NV - j ? v[k + 1] : 0.);
+                phr_s[buf][warp]  = hx;
+                pkey_s[buf][warp] = kmax;
+                pid_s[buf][warp]  = tid;
+              }
+            if constexpr (T == 32 * NW1)
+              __syncthreads();
+            else
+              asm volatile("bar.sync 1, %0;" ::"n"(32 * NW1) : "memory");
+            int      ww = 0;
+            unsigned kb = pkey_s[buf][0];
+#pragma unroll
+            for (int q = 1; q < NW1; ++q)
+              if (pkey_s[buf][q] > kb)
+                {
+                  kb = pkey_s[buf][q];
+                  ww = q;
+                }
+            const double2 *pr  = reinterpret_cast<const double2 *>(prow_s[buf][ww]);
+            const double   hr  = phr_s[buf][ww];
+            const bool     me  = tid == pid_s[buf][ww];
+            const double   l   = (used || me) ? 0. : -x0 * hr;
+#pragma unroll
+            for (int k = 0; k < NV; k += 2)
+              {
+                const double2 q = pr[k / 2];
+                if (k > 0)
+                  v[k - 1] = fma(l, q.x, v[k]);
+                v[k] = fma(l, q.y, v[k + 1]);
+              }
+            v[NV - 1] = (used || me) ? x0 : -l;
+            if (me)
+              {
+                used    = true;
+                pos     = j;
+                dinv[j] = hr;
+                perm[j] = tid;
+                if (!(fabs(x0) > 0.) || !isfinite(x0))
+                  sh_sing = 1;
+              }
+          }
+        if (pos >= 0)
+          {
+#pragma unroll
+            for (int c = 0; c < NSMAX; ++c)
+              if (c < Ns)
+                S[c * ldc + pos] = v[c];
+          }
+      }
+    __syncthreads();
+    constexpr int NB  = NP / 8;
+    const int     nbl = (Ns + 7) / 8; // blocks of eight rows in use
+    for (int c = tid; c < ncol; c += T)
+      {
+        double x[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k)
+          x[k] = k < Ns ? R[perm[k < NSMAX ? k : 0] * ncol + c] : 0.;
+        // unit lower factor: the current block in x[0 .. 7]; after a block
+        // the column is rotated by eight.  Entries beyond Ns take whatever
+        // follows a factor column and are never used.
+#pragma unroll 1
+        for (int g = 0; g < NB; ++g)
+          {
+            if (g < nbl)
+              {
+#pragma unroll
+                for (int jj = 0; jj < 8; ++jj)
+                  if (g * 8 + jj < Ns)
+                    {
+                      const double  y = -x[jj];
+                      const double *f = S + (g * 8 + jj) * ldc + g * 8;
+#pragma unroll
+                      for (int k = (jj + 1) / 2 * 2; k < 8; k += 2)
+                        {
+                          const double2 q = *reinterpret_cast<const double2 *>(f + k);
+                          if (k > jj)
+                            x[k] = fma(q.x, y, x[k]);
+                          x[k + 1] = fma(q.y, y, x[k + 1]);
+                        }
+#pragma unroll
+                      for (int b = 1; b < NB; ++b)
+                        if (b < nbl - g)
+#pragma unroll
+                          for (int k = b * 8; k < b * 8 + 8; k += 2)
+                            {
+                              const double2 q = *reinterpret_cast<const double2 *>(f + k);
+                              x[k]            = fma(q.x, y, x[k]);
+                              x[k + 1]        = fma(q.y, y, x[k + 1]);
+                            }
+                    }
+              }
+            double t[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              t[k] = x[k];
+#pragma unroll
+            for (int k = 8; k < NP; ++k)
+              x[k - 8] = x[k];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              x[NP - 8 + k] = t[k];
+          }
+        // upper factor: from the last block, the current one in the last
+        // eight registers
+#pragma unroll 1
+        for (int g = NB - 1; g >= 0; --g)
+          {
+            if (g < nbl)
+              {
+#pragma unroll
+                for (int jj = 7; jj >= 0; --jj)
+                  if (g * 8 + jj < Ns)
+                    {
+                      constexpr int o = NP - 8; // register of the block's first row
+                      x[o + jj] *= dinv[g * 8 + jj];
+                      const double  y = -x[o + jj];
+                      const double *f = S + (g * 8 + jj) * ldc + g * 8 - o; // row of register k: f[k]
+#pragma unroll
+                      for (int k = 0; k < jj; ++k)
+                        x[o + k] = fma(f[o + k], y, x[o + k]);
+#pragma unroll
+                      for (int b = 0; b < NB - 1; ++b)
+                        if (b >= NB - 1 - g)
+#pragma unroll
+                          for (int k = b * 8; k < b * 8 + 8; k += 2)
+                            {
+                              const double2 q = *reinterpret_cast<const double2 *>(f + k);
+                              x[k]            = fma(q.x, y, x[k]);
+                              x[k + 1]        = fma(q.y, y, x[k + 1]);
+                            }
+                    }
+              }
+            double t[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              t[k] = x[NP - 8 + k];
+#pragma unroll
+            for (int k = NP - 1; k >= 8; --k)
+              x[k] = x[k - 8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              x[k] = t[k];
+          }
+#pragma unroll
+        for (int k = 0; k < NSMAX; ++k)
+          if (k < Ns)
+            R[k * ncol + c] = x[k];
+      }
+    __syncthreads();
+  }
+
   // The body of the CTA-per-cell condensation: the CTA (T threads, a
-  // multiple of 32: CondenseTPB in condense2_kernel, fewer in the batched
+  // multiple of 32: condense2_threads in condense2_kernel, fewer in the batched
   // launch) works through the cells cell_begin, cell_begin + cell_step, ...
   // < cell_end with the workspace at smem (tables first when P.stage) and,
   // for R outside shared memory, the R slice `slot` of P.rscratch.
-  template <int DIM, int K, int T = CondenseTPB>
+  template <int DIM, int K, int T = condense2_threads(Dims<DIM, K>::nb)>
   __device__ __forceinline__ void
   condense2_cells(const KParams &P, double *smem, int64_t slot, int64_t cell_begin,
                   int64_t cell_end, int64_t cell_step)
@@ -822,105 +1035,82 @@ namespace ddhdg
         __syncthreads();
 
         // ------------------------------------------------ scalar system S
-        for (int idx = tid; idx < ncomp * ncomp * nb * nb; idx += T)
-          {
-            const int blk = idx / (nb * nb);
-            const int r_  = idx % (nb * nb);
-            const int a = r_ / nb, e = r_ % nb;
-            const int ci = blk / ncomp, cj = blk % ncomp;
-            const int pr = P.comps[ci] * 3 + P.comps[cj];
-            const double *alp = al + pr * nqc;
-            const double *kap = ka + pr * nqc;
-            const double *bep = be + pr * nqc * DIM;
-            const double *gap = ga + pr * Fq;
-            const double *rhp = rh + pr * Fq;
-            double        v   = 0.;
+        // Every block (test component, trial component) of S and R is a
+        // product over the channels on the FP64 tensor path: the A fragments
+        // are the coefficients times the test tables, the B fragments the
+        // trial tables; a warp per (block, eight rows).  The channels that
+        // vanish for a pair by the structure of the equations (densities
+        // couple to each other through the recombination only) are left out.
+        // An entry per thread took 42 % of the kernel (2D k = 3).
+        const int  g8 = lane >> 2, q4 = lane & 3;
+        constexpr int MTB = (nb + 7) / 8; // row tiles of a block
+        {
+          constexpr int NTB = (nb + 7) / 8;
+          for (int u = warp; u < ncomp * ncomp * MTB; u += NW)
+            {
+              const int  blk = u / MTB, mt = u % MTB;
+              const int  ci = blk / ncomp, cj = blk % ncomp;
+              const int  bi = P.comps[ci], bj = P.comps[cj], pr = bi * 3 + bj;
+              const int  a   = mt * 8 + g8;
+              const bool aok = a < nb;
+              double     d[NTB][2];
 #pragma unroll
-            for (int q = 0; q < nqc; ++q)
-              {
-                const double pe = phi_c[q * nb + e];
-                double       lt = alp[q] * TLc[q * nb + a];
-#pragma unroll
-                for (int s = 0; s < DIM; ++s)
+              for (int nt = 0; nt < NTB; ++nt)
+                d[nt][0] = d[nt][1] = 0.;
+              const auto add = [&](int nk, auto &&coef_tl, const double *rt) {
+                for (int k0 = 0; k0 < nk; k0 += 4)
                   {
-                    const double tg = TLg[(q * DIM + s) * nb + a];
-                    lt += bep[q * DIM + s] * tg;
-                    v += kap[q] * tg * RTk[(q * DIM + s) * nb + e];
+                    const int    j  = k0 + q4;
+                    const bool   ok = j < nk;
+                    const double av = (ok && aok) ? coef_tl(j) : 0.;
+#pragma unroll
+                    for (int nt = 0; nt < NTB; ++nt)
+                      {
+                        const int e = nt * 8 + g8;
+                        dmma8x8x4(d[nt][0], d[nt][1], av, (ok && e < nb) ? rt[j * nb + e] : 0.);
+                      }
                   }
-                v += lt * pe;
-              }
+              };
+              if (bi == 0 ? (bj == 0 ? phi_mode : !phi_mode) : bj > 0)
+                {
+                  const double *alp = al + pr * nqc, *bep = be + pr * nqc * DIM;
+                  add(
+                    nqc,
+                    [&](int j) {
+                      double v = alp[j] * TLc[j * nb + a];
+                      if (bi == bj)
 #pragma unroll
-            for (int fq = 0; fq < Fq; ++fq)
-              v += TLf[fq * nb + a] * (gap[fq] * phi_f[fq * nb + e] + rhp[fq] * RTr[fq * nb + e]);
-            S[(ci * nb + a) * ldS + cj * nb + e] = v;
-          }
-
-        // --------------------------------------------------------- R
-        // column 0: residual
-        for (int i = tid; i < Ns; i += T)
-          {
-            const int     ce = i / nb, a = i % nb;
-            const double *r0p = r0 + ce * nqc;
-            const double *r1p = r1 + ce * nqc * DIM;
-            const double *rfp = rf + ce * Fq;
-            double        v   = 0.;
+                        for (int s = 0; s < DIM; ++s)
+                          v += bep[j * DIM + s] * TLg[(j * DIM + s) * nb + a];
+                      return v;
+                    },
+                    phi_c);
+                }
+              if (bj == 0 || bi == bj)
+                {
+                  const double *kap = ka + pr * nqc, *rhp = rh + pr * Fq;
+                  add(nqc * DIM, [&](int j) { return kap[j / DIM] * TLg[j * nb + a]; }, RTk);
+                  add(Fq, [&](int j) { return rhp[j] * TLf[j * nb + a]; }, RTr);
+                }
+              if (bi == bj)
+                {
+                  const double *gap = ga + pr * Fq;
+                  add(Fq, [&](int j) { return gap[j] * TLf[j * nb + a]; }, phi_f);
+                }
+              if (aok)
 #pragma unroll
-            for (int q = 0; q < nqc; ++q)
-              {
-                v += TLc[q * nb + a] * r0p[q];
+                for (int nt = 0; nt < NTB; ++nt)
 #pragma unroll
-                for (int s = 0; s < DIM; ++s)
-                  v += TLg[(q * DIM + s) * nb + a] * r1p[q * DIM + s];
-              }
-#pragma unroll
-            for (int fq = 0; fq < Fq; ++fq)
-              v += TLf[fq * nb + a] * rfp[fq];
-            R[i * ncol] = v;
-          }
-        // trace columns: ct_z - A_zW Q  (and the drift parts)
-        for (int idx = tid; idx < Ns * Nt; idx += T)
-          {
-            const int i = idx / Nt, t = idx % Nt;
-            const int ci = i / nb, a = i % nb;
-            const int ft = t / (ncomp * nf), ct = (t / nf) % ncomp, mt = t % nf;
-            const int pr = P.comps[ci] * 3 + P.comps[ct];
-            const int tq = ft * nf + mt;
-            const double *kap = ka + pr * nqc;
-            const double *rhp = rh + pr * Fq;
-            double        v   = 0., vd = 0.;
-#pragma unroll
-            for (int q = 0; q < nqc; ++q)
-              {
-                double gk = 0.;
-#pragma unroll
-                for (int s = 0; s < DIM; ++s)
-                  gk += TLg[(q * DIM + s) * nb + a] * RQk[(q * DIM + s) * Ft + tq];
-                v -= kap[q] * gk;
-              }
-#pragma unroll
-            for (int fq = 0; fq < Fq; ++fq)
-              v -= rhp[fq] * TLf[fq * nb + a] * RQr[fq * Ft + tq];
-            if (ci == ct)
-              {
-                const int b = P.comps[ci];
-#pragma unroll
-                for (int qf = 0; qf < nqf; ++qf)
-                  {
-                    const int    fq = ft * nqf + qf;
-                    const double tx = TLf[fq * nb + a] * xi[qf * nf + mt];
-                    v += ctc[b * Fq + fq] * tx;
-                    vd += ctd[b * Fq + fq] * tx;
-                  }
-              }
-            R[i * ncol + 1 + t] = v;
-            if (two)
-              R[i * ncol + 1 + Nt + t] = vd;
-          }
+                  for (int e = 0; e < 2; ++e)
+                    if (nt * 8 + 2 * q4 + e < nb)
+                      S[(ci * nb + a) * ldS + cj * nb + nt * 8 + 2 * q4 + e] = d[nt][e];
+            }
+        }
         if (tid == 0)
           sh_sing = 0;
         __syncthreads();
-
-        // -------------------------- equilibrate rows, LU with partial pivoting
+        // row equilibration of S; the factors wait in rhsA for R
+        double *scl = rhsA;
         for (int i = warp; i < Ns; i += NW)
           {
             double mx = 0.;
@@ -932,11 +1122,108 @@ namespace ddhdg
             const double sc = (mx > 0.) ? 1. / mx : 1.;
             for (int j = lane; j < Ns; j += 32)
               S[i * ldS + j] *= sc;
-            for (int c = lane; c < ncol; c += 32)
-              R[i * ncol + c] *= sc;
+            if (lane == 0)
+              scl[i] = sc;
           }
         __syncthreads();
-        cta_lu_solve<T, 3 * nb>(S, ldS, R, ncol, Ns, sh_p8, sh_sing);
+
+        // --------------------------------------- R, rows scaled like S's
+        // column 0: residual
+        for (int i = tid; i < Ns; i += T)
+          {
+            const int     ce = i / nb, a = i % nb;
+            const double *r0p = r0 + ce * nqc;
+            const double *r1p = r1 + ce * nqc * DIM;
+            const double *rfp = rf + ce * Fq;
+            double        v   = 0.;
+#pragma unroll 4
+            for (int q = 0; q < nqc; ++q)
+              {
+                v += TLc[q * nb + a] * r0p[q];
+#pragma unroll
+                for (int s = 0; s < DIM; ++s)
+                  v += TLg[(q * DIM + s) * nb + a] * r1p[q * DIM + s];
+              }
+#pragma unroll 4
+            for (int fq = 0; fq < Fq; ++fq)
+              v += TLf[fq * nb + a] * rfp[fq];
+            R[i * ncol] = v * scl[i];
+          }
+        // trace columns: ct_z - A_zW Q  (and the drift parts)
+        {
+          constexpr int NTR = (Ft + 7) / 8;
+          for (int u = warp; u < ncomp * ncomp * MTB; u += NW)
+            {
+              const int    blk = u / MTB, mt = u % MTB;
+              const int    ci = blk / ncomp, ct = blk % ncomp;
+              const int    bi = P.comps[ci], bt = P.comps[ct], pr = bi * 3 + bt;
+              const int    a   = mt * 8 + g8;
+              const bool   aok = a < nb;
+              const double sc  = aok ? scl[ci * nb + a] : 0.;
+              double       d[NTR][2];
+#pragma unroll
+              for (int nt = 0; nt < NTR; ++nt)
+                d[nt][0] = d[nt][1] = 0.;
+              const auto add = [&](int nk, auto &&coef_tl, auto &&rt) {
+                for (int k0 = 0; k0 < nk; k0 += 4)
+                  {
+                    const int    j  = k0 + q4;
+                    const bool   ok = j < nk;
+                    const double av = (ok && aok) ? coef_tl(j) : 0.;
+#pragma unroll
+                    for (int nt = 0; nt < NTR; ++nt)
+                      {
+                        const int t = nt * 8 + g8;
+                        dmma8x8x4(d[nt][0], d[nt][1], av, (ok && t < Ft) ? rt(j, t) : 0.);
+                      }
+                  }
+              };
+              const auto store = [&](int off) {
+                if (aok)
+#pragma unroll
+                  for (int nt = 0; nt < NTR; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                      {
+                        const int t = nt * 8 + 2 * q4 + e;
+                        if (t < Ft)
+                          R[(ci * nb + a) * ncol + off + ((t / nf) * ncomp + ct) * nf + t % nf] = d[nt][e] * sc;
+                      }
+              };
+              // the face's own trace values: coefficient x test table against
+              // the face basis, face by face
+              const auto face = [&](int j, int t) {
+                return j / nqf == t / nf ? xi[(j % nqf) * nf + t % nf] : 0.;
+              };
+              if (bt == 0 || bi == bt)
+                {
+                  const double *kap = ka + pr * nqc, *rhp = rh + pr * Fq;
+                  add(nqc * DIM, [&](int j) { return -kap[j / DIM] * TLg[j * nb + a]; },
+                      [&](int j, int t) { return RQk[j * Ft + t]; });
+                  add(Fq, [&](int j) { return -rhp[j] * TLf[j * nb + a]; },
+                      [&](int j, int t) { return RQr[j * Ft + t]; });
+                }
+              if (ci == ct)
+                add(Fq, [&](int j) { return ctc[bi * Fq + j] * TLf[j * nb + a]; }, face);
+              store(1);
+              if (two)
+                {
+#pragma unroll
+                  for (int nt = 0; nt < NTR; ++nt)
+                    d[nt][0] = d[nt][1] = 0.;
+                  if (ci == ct)
+                    add(Fq, [&](int j) { return ctd[bi * Fq + j] * TLf[j * nb + a]; }, face);
+                  store(1 + Nt);
+                }
+            }
+        }
+        __syncthreads();
+
+        // -------------------------------------------- LU with partial pivoting
+        if constexpr (3 * nb > 64)
+          cta_lu_solve<T, 3 * nb>(S, R, ncol, Ns, sh_sing);
+        else
+          cta_lu_blocked<T, 3 * nb>(S, ldS, R, ncol, Ns, sh_p8, sh_sing);
         if (tid == 0 && sh_sing)
           atomicExch(P.status, 3);
 
@@ -1006,7 +1293,7 @@ namespace ddhdg
                           if (two && col > 0)
                             bv += R[j * ncol + col + Nt];
                         }
-                      cta_dmma8x8x4(d[nt][0], d[nt][1], av, bv);
+                      dmma8x8x4(d[nt][0], d[nt][1], av, bv);
                     }
                 }
               const bool rok   = iok && dfl[ii] == 0.;
@@ -1081,10 +1368,10 @@ namespace ddhdg
   }
 
   template <int DIM, int K>
-  __global__ void __launch_bounds__(CondenseTPB)
+  __global__ void __launch_bounds__(condense2_threads(Dims<DIM, K>::nb))
   condense2_kernel(const KParams P)
   {
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];
     condense2_cells<DIM, K>(P, smem, blockIdx.x, P.cell0 + blockIdx.x, P.ncells, gridDim.x);
   }
 } // namespace ddhdg

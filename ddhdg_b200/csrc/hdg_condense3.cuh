@@ -25,7 +25,15 @@
 
 namespace ddhdg
 {
-  constexpr int Condense3MaxWPB = 8; // warps (cells) per CTA at most
+  // warps (cells) per CTA at most, by the nodes of a cell and the bytes of
+  // the Jacobian type: FP64 eight with 255 registers (2D k = 2, 3D k = 1),
+  // sixteen with 128 where the bodies need no more; mixed eight, two CTAs per
+  // SM
+  __host__ __device__ constexpr int
+  condense3_max_warps(int nb, int jb)
+  {
+    return jb == 8 && nb <= 4 ? 16 : 8;
+  }
 
   // row stride of the staged S^-1 (>= its padded width, = 4 mod 16 doubles:
   // the A-fragment loads of a half warp hit 16 different 8-byte banks)
@@ -1160,11 +1168,11 @@ namespace ddhdg
   }
 
   template <int DIM, int K, typename JT = double>
-  __global__ void __launch_bounds__(Condense3MaxWPB * 32, sizeof(JT) == 8 ? 1 : 2)
+  __global__ void __launch_bounds__(condense3_max_warps(Dims<DIM, K>::nb, sizeof(JT)) * 32, sizeof(JT) == 8 ? 1 : 2)
   condense3_kernel(const KParams P, const __grid_constant__ CTab<DIM, K> C)
   {
     extern __shared__ __align__(16) double smem[];
-    __shared__ int    piv3[Condense3MaxWPB][3 * Dims<DIM, K>::nb];
+    __shared__ int    piv3[condense3_max_warps(Dims<DIM, K>::nb, sizeof(JT))][3 * Dims<DIM, K>::nb];
     __shared__ double rqr_s[CTab<DIM, K>::Fq * CTab<DIM, K>::Ft];
     for (int i = threadIdx.x; i < CTab<DIM, K>::Fq * CTab<DIM, K>::Ft; i += blockDim.x)
       rqr_s[i] = P.tables[P.to.RQr + i];

@@ -1,0 +1,70 @@
+// Condensation and reconstruction kernels of one dimension (DDHDG_DIM).
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "hdg_launch.h"
+
+namespace ddhdg
+{
+  namespace
+  {
+    template <int D, int K, typename JT>
+    void
+    launch_condense(const Tables &T, const KParams &P, int grid, int threads, size_t smem, cudaStream_t s)
+    {
+      if constexpr (3 * Dims<D, K>::nb <= 32)
+        {
+          CTab<D, K> C;
+          fill_ctab(T, C);
+          condense3_kernel<D, K, JT><<<grid, threads, smem, s>>>(P, C);
+        }
+      else
+        condense2_kernel<D, K><<<grid, threads, smem, s>>>(P);
+    }
+
+    template <int D, int K>
+    bool
+    pick(CondenseKernel &cf, ReconstructFn &rf, bool mixed)
+    {
+      // register kernel when one lane can own one row of the scalar system,
+      // CTA-per-cell shared-memory kernel otherwise
+      rf = reconstruct_kernel<D, K>;
+      if constexpr (3 * Dims<D, K>::nb <= 32)
+        {
+          if (mixed)
+            {
+              cf.fn     = reinterpret_cast<const void *>(condense3_kernel<D, K, float>);
+              cf.launch = launch_condense<D, K, float>;
+            }
+          else
+            {
+              cf.fn     = reinterpret_cast<const void *>(condense3_kernel<D, K, double>);
+              cf.launch = launch_condense<D, K, double>;
+            }
+          return true;
+        }
+      else
+        {
+          cf.fn     = reinterpret_cast<const void *>(condense2_kernel<D, K>);
+          cf.launch = launch_condense<D, K, double>;
+          return !mixed;
+        }
+    }
+  } // namespace
+
+  template <>
+  bool
+  condense_kernels<DDHDG_DIM>(int k, CondenseKernel &cf, ReconstructFn &rf, bool mixed)
+  {
+    if (k == 1)
+      return pick<DDHDG_DIM, 1>(cf, rf, mixed);
+    if (k == 2)
+      return pick<DDHDG_DIM, 2>(cf, rf, mixed);
+#if DDHDG_DIM < 3
+    if (k == 3)
+      return pick<DDHDG_DIM, 3>(cf, rf, mixed);
+#endif
+    return false;
+  }
+} // namespace ddhdg
