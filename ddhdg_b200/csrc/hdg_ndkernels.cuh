@@ -169,6 +169,18 @@ namespace ddhdg
     return (unsigned)((unsigned long long)__double_as_longlong(fabs(x)) >> 32) + 1u;
   }
 
+  // 1 / x by Newton's iteration from the hardware's approximation: no branch,
+  // so that it overlaps the pivot search; 0 for x = 0
+  __device__ __forceinline__ double
+  nd_reciprocal(double x)
+  {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(r, fma(-x, r, 1.), r);
+    r = fma(r, fma(-x, r, 1.), r);
+    return x != 0. ? r : 0.;
+  }
+
   // ------------------------------------------------------------ small fronts
   // nE <= NEM <= 36: the whole elimination of a front in one CTA.
   // - F_EE goes into the registers of one warp (two for NEM > 32), a row per
@@ -588,6 +600,21 @@ namespace ddhdg
   constexpr int NDPanelG  = 8;             // columns per group
   constexpr int NDPanelN  = NDPanel / NDPanelG;
 
+  // pivot key of a panel row: sign-free high word of the candidate down to 11
+  // mantissa bits (the pivot is within 2^-11 of the largest), plus one, and
+  // the thread, the first one winning ties
+  __device__ __forceinline__ unsigned
+  nd_panel_key(double x, int thread)
+  {
+    const unsigned hi = (unsigned)((unsigned long long)__double_as_longlong(fabs(x)) >> 32);
+    return (((hi >> 9) + 1u) << 9) | (unsigned)(NDPanelT - 1 - thread);
+  }
+  __device__ __forceinline__ int
+  nd_panel_key_row(unsigned key)
+  {
+    return NDPanelT - 1 - (int)(key & (NDPanelT - 1));
+  }
+
   template <int CL>
   struct NDPanelShared
   {
@@ -599,7 +626,6 @@ namespace ddhdg
     double   whr[2][NW], chr[2][CL]; // reciprocal pivots
     double   rd[NDPanel];            // reciprocals of the diagonal of U (1 beyond w)
     unsigned wkey[2][NW], ckey[2][CL];
-    int      wid[2][NW], cid[2][CL];
     int      ppos[NDPanel]; // list positions of the pivot rows
   };
 
@@ -608,7 +634,7 @@ namespace ddhdg
   template <int CL>
   __device__ __forceinline__ void
   nd_panel_group(double (&v)[NDPanel], NDPanelShared<CL> &S, int j0, int nact, int w, int t, int rank, bool &used,
-                 int &mypos, int *sing)
+                 int &mypos)
   {
     namespace cg   = cooperative_groups;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -618,11 +644,10 @@ namespace ddhdg
         constexpr int  PK   = 2; // columns per 16-byte access
         const int      buf  = jj & 1;
         const double   x0   = v[jj];
-        const unsigned key  = used ? 0u : nd_pivot_key(x0);
-        const double   hx   = (x0 != 0.) ? 1. / x0 : 0.; // overlaps the reduction
+        const unsigned key  = used ? 0u : nd_panel_key(x0, threadIdx.x);
+        const double   hx   = nd_reciprocal(x0);
         const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
-        const int      src  = __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1;
-        if (lane == src)
+        if (key == kmax && key != 0u)
           {
             double2 *dst = reinterpret_cast<double2 *>(S.wrow[buf][warp]);
 #pragma unroll
@@ -634,17 +659,16 @@ namespace ddhdg
 #pragma unroll
                 for (int k = b * NDPanelG; k < (b + 1) * NDPanelG; k += PK)
                   dst[k / PK] = make_double2(v[k], v[k + 1]);
-            S.whr[buf][warp]  = hx;
-            S.wkey[buf][warp] = kmax;
-            S.wid[buf][warp]  = t;
+            S.whr[buf][warp] = hx;
           }
+        if (lane == 0)
+          S.wkey[buf][warp] = kmax;
         __syncthreads();
-        const unsigned k2 = lane < nw ? S.wkey[buf][lane] : 0u;
-        const unsigned m2 = __reduce_max_sync(0xffffffffu, k2);
-        const int      ww = __ffs(__ballot_sync(0xffffffffu, lane < nw && k2 == m2)) - 1;
-        const double  *prow = S.wrow[buf][ww];
-        double         hr   = S.whr[buf][ww];
-        int            pid  = S.wid[buf][ww];
+        const unsigned m2   = __reduce_max_sync(0xffffffffu, lane < nw ? S.wkey[buf][lane] : 0u);
+        const int      tw   = nd_panel_key_row(m2); // thread of the CTA's candidate
+        const double  *prow = S.wrow[buf][tw >> 5];
+        double         hr   = S.whr[buf][tw >> 5];
+        int            pid  = rank * (int)blockDim.x + tw;
         if (CL > 1)
           {
             cg::cluster_group cl = cg::this_cluster();
@@ -655,7 +679,6 @@ namespace ddhdg
                 if (lane == 0)
                   {
                     *cl.map_shared_rank(&S.ckey[buf][rank], warp) = m2;
-                    *cl.map_shared_rank(&S.cid[buf][rank], warp)  = pid;
                     *cl.map_shared_rank(&S.chr[buf][rank], warp)  = hr;
                   }
               }
@@ -665,7 +688,7 @@ namespace ddhdg
             const int      cc = __ffs(__ballot_sync(0xffffffffu, lane < CL && k3 == m3)) - 1;
             prow              = S.crow[buf][cc];
             hr                = S.chr[buf][cc];
-            pid               = S.cid[buf][cc];
+            pid               = cc * (int)blockDim.x + nd_panel_key_row(m3);
           }
         const bool    me = !used && t == pid;
         const double  l  = (used || me) ? 0. : -x0 * hr;
@@ -694,8 +717,6 @@ namespace ddhdg
           {
             used  = true;
             mypos = j0 + jj;
-            if (!(fabs(x0) > 0.) || !isfinite(x0))
-              atomicExch(sing, 1);
           }
         if (threadIdx.x == 0 && j0 + jj < w)
           {
@@ -751,7 +772,7 @@ namespace ddhdg
       __syncthreads();
 #pragma unroll 1
     for (int g = 0; g < NDPanelN; ++g)
-      nd_panel_group<CL>(v, S, g * NDPanelG, NDPanelN - g, w, t, rank, used, mypos, sing);
+      nd_panel_group<CL>(v, S, g * NDPanelG, NDPanelN - g, w, t, rank, used, mypos);
     if (mypos >= 0)
       {
         double *d0 = &S.LU[0][0][mypos], *d1 = &S.LU[1][NDPanel - 1][NDPanel - 1 - mypos];
@@ -771,6 +792,8 @@ namespace ddhdg
       cg::this_cluster().sync(); // also: no CTA's shared memory is written after this
     else
       __syncthreads();
+    if (rank == 0 && tid < w && (S.rd[tid] == 0. || !isfinite(S.rd[tid])))
+      atomicExch(sing, 1); // a zero, subnormal or non-finite pivot
     if (mypos >= 0)
       perm[n.poff + k0 + mypos] = row;
     else if (has)
