@@ -444,7 +444,7 @@ namespace ddhdg
             if constexpr (T == 32 * NW1)
               __syncthreads();
             else
-              asm volatile("bar.sync 1, %0;" ::"n"(32 * NW1) : "memory");
+              asm volatile("barrier.sync 1, %0;" ::"n"(32 * NW1) : "memory");
             int      ww = 0;
             unsigned kb = pkey_s[buf][0];
 #pragma unroll

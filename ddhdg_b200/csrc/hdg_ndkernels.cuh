@@ -169,6 +169,13 @@ namespace ddhdg
     return (unsigned)((unsigned long long)__double_as_longlong(fabs(x)) >> 32) + 1u;
   }
 
+  // barrier of a whole cluster, for warps that need not be converged
+  __device__ __forceinline__ void
+  nd_cluster_sync()
+  {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  }
+
   // 1 / x by Newton's iteration from the hardware's approximation: no branch,
   // so that it overlaps the pivot search; 0 for x = 0
   __device__ __forceinline__ double
@@ -271,31 +278,31 @@ namespace ddhdg
       }
     const bool cells = LEAF || n.ccell[0] >= 0 || n.ccell[1] >= 0;
     __syncthreads();
-    // entry of a row (pointer, scale, column offset of its own position)
-    const auto entry = [&](const double *rp, double rs, int own, int co) -> double {
+    // value of an entry from what its place holds: row scale, column offsets
+    // of the row's own position and of the entry
+    const auto entry = [&](double x, double rs, int own, int co) -> double {
       if (cells && rs == 0.)
         return own == co ? 1. : 0.;
-      return rs * rp[co];
+      return rs * x;
     };
-    // right-hand side of a row of child s
-    const auto rhs = [&](int s, const double *rp, double rs, int own) -> double {
+    // place of the right-hand side of a row of child s (Dirichlet rows: their
+    // value, unscaled)
+    const auto rhs_at = [&](int s, const double *rp, double rs, int own) -> const double * {
       const int64_t cell = LEAF ? n.cell : (s ? n.ccell[1] : n.ccell[0]);
       if (cell >= 0)
-        {
-          const int64_t r = cell * C.Nt + own;
-          return rs == 0. ? C.dval[r] : rs * C.rhs[r];
-        }
-      return rp[(int64_t)(s ? n.cnK[1] : n.cnK[0]) * (s ? n.cld[1] : n.cld[0])];
+        return (rs == 0. ? C.dval : C.rhs) + cell * C.Nt + own;
+      return rp + (int64_t)(s ? n.cnK[1] : n.cnK[0]) * (s ? n.cld[1] : n.cld[0]);
     };
+    const auto rhs_scale = [&](double rs) { return cells && rs == 0. ? 1. : rs; };
     for (int idx = tid; idx < NEM * NEM; idx += T)
       {
         const int i = idx % NEM, c = idx / NEM;
         double    x = (i == c) ? 1. : 0.;
         if (i < nE && c < nE)
           {
-            x = entry(erp[i], ers[i], eco[i], eco[c]);
+            x = entry(erp[i][eco[c]], ers[i], eco[i], eco[c]);
             if (!LEAF)
-              x += entry(erp[NEM + i], ers[NEM + i], eco[NEM + i], eco[NEM + c]);
+              x += entry(erp[NEM + i][eco[NEM + c]], ers[NEM + i], eco[NEM + i], eco[NEM + c]);
           }
         LU[idx] = x;
       }
@@ -316,7 +323,7 @@ namespace ddhdg
             const int      buf  = j & 1;
             const double   x0   = v[0];
             const unsigned key  = used ? 0u : nd_pivot_key(x0);
-            const double   hx   = (x0 != 0.) ? 1. / x0 : 0.; // overlaps the reduction
+            const double   hx   = nd_reciprocal(x0); // overlaps the reduction
             const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
             const int      src  = __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1;
             if (lane == src)
@@ -331,7 +338,7 @@ namespace ddhdg
                 pid_s[buf][warp]  = tid;
               }
             if (NLW > 1)
-              asm volatile("bar.sync 1, 64;" ::: "memory");
+              asm volatile("barrier.sync 1, 64;" ::: "memory");
             else
               __syncwarp();
             const int     ww   = (NLW > 1 && pkey_s[buf][NLW - 1] > pkey_s[buf][0]) ? NLW - 1 : 0;
@@ -350,7 +357,7 @@ namespace ddhdg
                 pos     = j;
                 dinv[j] = hr;
                 perm[j] = tid;
-                bad |= !(fabs(x0) > 0.) || !isfinite(x0);
+                bad |= hr == 0. || !isfinite(hr); // zero, subnormal or non-finite pivot
               }
           }
 #pragma unroll 1
@@ -380,31 +387,58 @@ namespace ddhdg
     else
       {
         const int t0 = tid - 32 * NLW, TT = T - 32 * NLW;
-        for (int idx = t0; idx < NEM * (nK + 1); idx += TT)
+        // GU entries in flight per thread: their loads are unconditional, so
+        // that they do not wait for each other
+        constexpr int GU = 4;
+        const int     nB = nE * nK;
+        for (int i0 = t0; i0 < nB; i0 += GU * TT)
           {
-            const int i = idx % NEM, c = idx / NEM;
-            double    x = 0.;
-            if (i < nE)
+            double x[GU];
+#pragma unroll
+            for (int u = 0; u < GU; ++u)
               {
-                if (c == nK)
-                  {
-                    x = rhs(0, erp[i], ers[i], eco[i]);
-                    if (!LEAF)
-                      x += rhs(1, erp[NEM + i], ers[NEM + i], eco[NEM + i]);
-                  }
-                else
-                  {
-                    const int e = kid[c] * NEM + i;
-                    x           = entry(erp[e], ers[e], eco[e], kco[c]);
-                  }
+                const int idx = min(i0 + u * TT, nB - 1), i = idx % nE, c = idx / nE;
+                const int e   = kid[c] * NEM + i;
+                x[u]          = entry(erp[e][kco[c]], ers[e], eco[e], kco[c]);
               }
-            Bs[c * LDW + i] = x;
+#pragma unroll
+            for (int u = 0; u < GU; ++u)
+              {
+                const int idx = i0 + u * TT;
+                if (idx < nB)
+                  Bs[(idx / nE) * LDW + idx % nE] = x[u];
+              }
           }
-        for (int idx = t0; idx < nK * NEM; idx += TT)
+        for (int i0 = t0; i0 < nB; i0 += GU * TT)
           {
-            const int r = idx % nK, j = idx / nK;
-            Ks[r * LDW + j] = j < nE ? -entry(krp[r], krs[r], kco[r], eco[kid[r] * NEM + j]) : 0.;
+            double x[GU];
+#pragma unroll
+            for (int u = 0; u < GU; ++u)
+              {
+                const int idx = min(i0 + u * TT, nB - 1), r = idx % nK, j = idx / nK;
+                const int co  = eco[kid[r] * NEM + j];
+                x[u]          = entry(krp[r][co], krs[r], kco[r], co);
+              }
+#pragma unroll
+            for (int u = 0; u < GU; ++u)
+              {
+                const int idx = i0 + u * TT;
+                if (idx < nB)
+                  Ks[(idx % nK) * LDW + idx / nK] = -x[u];
+              }
           }
+        for (int i = t0; i < nE; i += TT)
+          {
+            double x = rhs_scale(ers[i]) * *rhs_at(0, erp[i], ers[i], eco[i]);
+            if (!LEAF)
+              x += rhs_scale(ers[NEM + i]) * *rhs_at(1, erp[NEM + i], ers[NEM + i], eco[NEM + i]);
+            Bs[nK * LDW + i] = x;
+          }
+        // beyond nE
+        for (int idx = t0; idx < (NEM - nE) * (nK + 1); idx += TT)
+          Bs[idx / (NEM - nE) * LDW + nE + idx % (NEM - nE)] = 0.;
+        for (int idx = t0; idx < (NEM - nE) * nK; idx += TT)
+          Ks[idx / (NEM - nE) * LDW + nE + idx % (NEM - nE)] = 0.;
       }
     __syncthreads();
     // W, a thread per column
@@ -463,7 +497,7 @@ namespace ddhdg
         const int r0 = (tile % rt) * 16, c0 = (tile / rt) * 32;
         double    acc[2][4][2];
         {
-          const double *rp[2];
+          const double *rp[2], *rr[2];
           double        rs[2];
           int           rk[2], ro[2];
 #pragma unroll
@@ -474,23 +508,24 @@ namespace ddhdg
               rs[i]       = krs[r];
               rk[i]       = kid[r];
               ro[i]       = kco[r];
+              rr[i]       = rhs_at(rk[i], rp[i], rs[i], ro[i]);
             }
 #pragma unroll
           for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int e = 0; e < 2; ++e)
               {
-                const int c  = c0 + j * 8 + 2 * tq + e;
-                const int ck = c < nK ? kid[c] : -1, co = c < nK ? kco[c] : 0;
+                const int c  = c0 + j * 8 + 2 * tq + e, cc = min(c, nK - 1);
+                const int ck = c < nK ? kid[cc] : -1, co = kco[cc];
+                // every load is made (behind branches they would wait for
+                // each other), from the row's right-hand side where the entry
+                // is zero
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
                   {
-                    double x = 0.;
-                    if (ck == rk[i])
-                      x = entry(rp[i], rs[i], ro[i], co);
-                    else if (c == nK)
-                      x = rhs(rk[i], rp[i], rs[i], ro[i]);
-                    acc[i][j][e] = x;
+                    const bool   in = ck == rk[i];
+                    const double x  = *(in ? rp[i] + co : rr[i]);
+                    acc[i][j][e]    = in ? entry(x, rs[i], ro[i], co) : (c == nK ? rhs_scale(rs[i]) * x : 0.);
                   }
               }
         }
@@ -537,6 +572,7 @@ namespace ddhdg
     for (int j = blockIdx.x; j < n.nE; j += gridDim.x)
       {
         double *A = ecols + n.eoff + (int64_t)j * n.ld;
+#pragma unroll 4
         for (int i = threadIdx.x; i < n.ld; i += 256)
           {
             double x = 0.; // the pad rows stay zero
@@ -564,6 +600,7 @@ namespace ddhdg
       return;
     const NDFront  F{n, C, maps + n.map, fronts};
     const int32_t *perm = perm_all + n.poff;
+#pragma unroll 4
     for (int idx = threadIdx.x; idx < nc * nE; idx += 256)
       sm[idx] = F.EK(idx % nE, c0 + idx / nE);
     __syncthreads();
@@ -641,6 +678,8 @@ namespace ddhdg
 #pragma unroll
     for (int jj = 0; jj < NDPanelG; ++jj)
       {
+        if (j0 + jj >= w)
+          break; // no rows are left (the same for every CTA of the cluster)
         constexpr int  PK   = 2; // columns per 16-byte access
         const int      buf  = jj & 1;
         const double   x0   = v[jj];
@@ -682,7 +721,7 @@ namespace ddhdg
                     *cl.map_shared_rank(&S.chr[buf][rank], warp)  = hr;
                   }
               }
-            cl.sync();
+            nd_cluster_sync();
             const unsigned k3 = lane < CL ? S.ckey[buf][lane] : 0u;
             const unsigned m3 = __reduce_max_sync(0xffffffffu, k3);
             const int      cc = __ffs(__ballot_sync(0xffffffffu, lane < CL && k3 == m3)) - 1;
@@ -718,7 +757,7 @@ namespace ddhdg
             used  = true;
             mypos = j0 + jj;
           }
-        if (threadIdx.x == 0 && j0 + jj < w)
+        if (threadIdx.x == 0)
           {
             S.ppos[j0 + jj] = pid;
             S.rd[j0 + jj]   = hr;
@@ -767,7 +806,7 @@ namespace ddhdg
     if (tid < NDPanel)
       S.rd[tid] = 1.;
     if (CL > 1)
-      cg::this_cluster().sync(); // every CTA of the cluster runs before its shared memory is written
+      nd_cluster_sync(); // every CTA of the cluster runs before its shared memory is written
     else
       __syncthreads();
 #pragma unroll 1
@@ -789,7 +828,7 @@ namespace ddhdg
           }
       }
     if (CL > 1)
-      cg::this_cluster().sync(); // also: no CTA's shared memory is written after this
+      nd_cluster_sync(); // also: no CTA's shared memory is written after this
     else
       __syncthreads();
     if (rank == 0 && tid < w && (S.rd[tid] == 0. || !isfinite(S.rd[tid])))
@@ -1374,10 +1413,12 @@ namespace ddhdg
         constexpr int  KM = (1 << NDKidBit) - 1;
         const double  *rp[4];
         int            rk[4];
+        int64_t        rr[4]; // offset of the right-hand-side column
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           {
             const int k = km[min(m0 + wm + i * 8 + g, m - 1)];
+            rr[i]       = (int64_t)((k >> NDKidBit) ? n.cnK[1] : n.cnK[0]) * ((k >> NDKidBit) ? n.cld[1] : n.cld[0]);
             rk[i]       = k >> NDKidBit;
             rp[i]       = fronts + (rk[i] ? n.coff[1] : n.coff[0]) + (rk[i] ? n.cEp[1] : n.cEp[0]) + (k & KM);
           }
@@ -1390,15 +1431,15 @@ namespace ddhdg
               const int     k  = km[min(c, n.nK - 1)];
               const int     ck = c < n.nK ? k >> NDKidBit : -1;
               const int64_t co = (int64_t)(k & KM) * (ck > 0 ? n.cld[1] : n.cld[0]);
+              // every load is made, from a fixed place where the entry is
+              // zero: behind branches the loads would wait for each other
 #pragma unroll
               for (int i = 0; i < 4; ++i)
                 {
-                  double x = 0.;
-                  if (ck == rk[i])
-                    x = rp[i][co];
-                  else if (c == n.nK)
-                    x = rp[i][(int64_t)(rk[i] ? n.cnK[1] : n.cnK[0]) * (rk[i] ? n.cld[1] : n.cld[0])];
-                  acc[i][j][e] = x;
+                  const bool    in  = ck == rk[i] || c == n.nK;
+                  const int64_t off = c == n.nK ? rr[i] : co;
+                  const double  x   = *(in ? rp[i] + off : fronts);
+                  acc[i][j][e]      = in ? x : 0.;
                 }
             }
       }
