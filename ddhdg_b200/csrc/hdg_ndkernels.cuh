@@ -1158,38 +1158,47 @@ namespace ddhdg
   // the factors stream through a ring of cp.async stages, the diagonal blocks
   // as their inverses, all products on the FP64 tensor path.  Bound by the
   // factors' L2 reads and the tensor path; one read and one write of B.
-  constexpr int NDSolveCols   = 32;
-  constexpr int NDSolveStages = 4;
+  // CT columns per CTA: 64 where there are enough tiles to fill the GPU (half
+  // the factor reads and twice the products per barrier), else 32.
+  constexpr int NDSolveStages = 3;
 
-  __host__ __device__ inline size_t
-  nd_solve_smem(int bs)
+  __host__ __device__ constexpr int
+  nd_solve_rows(int CT) // rows of a column tile that fit in shared memory
   {
-    const int rows = (bs + NDPanel - 1) / NDPanel * NDPanel;
-    return ((size_t)NDSolveCols * (rows + 4) + (size_t)NDSolveStages * NDPanel * NDPanelLd) * sizeof(double);
+    return CT == 64 ? 288 : 576;
   }
 
+  __host__ __device__ inline size_t
+  nd_solve_smem(int CT, int bs)
+  {
+    const int rows = (bs + NDPanel - 1) / NDPanel * NDPanel;
+    return ((size_t)CT * (rows + 4) + (size_t)NDSolveStages * NDPanel * NDPanelLd) * sizeof(double);
+  }
+
+  template <int CT>
   __global__ void __launch_bounds__(256)
   nd_solve_kernel(const NDNode *nodes, int b0, int bs, int dir, const double *luf, const double *tinv,
                   double *fronts)
   {
     extern __shared__ __align__(16) double sm[];
     const NDNode &n  = nodes[blockIdx.y];
-    const int     c0 = blockIdx.x * NDSolveCols, nc = min(NDSolveCols, n.nK + 1 - c0);
+    const int     c0 = blockIdx.x * CT, nc = min(CT, n.nK + 1 - c0);
     const int     nr = min(bs, n.nE - b0);
     if (nc <= 0 || nr <= 0)
       return;
     const int     nblk = (nr + NDPanel - 1) / NDPanel;
     const int     ldb  = (bs + NDPanel - 1) / NDPanel * NDPanel + 4;
     double       *Bs   = sm;                                   // [column][row]
-    double       *Ts   = sm + (size_t)NDSolveCols * ldb;       // stages of [column][row] blocks
+    double       *Ts   = sm + (size_t)CT * ldb;               // stages of [column][row] blocks
     const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int     g = lane >> 2, q = lane & 3;
-    const int     mt = warp & 3, nt = (warp >> 2) * 2;
+    constexpr int NT = CT / 16; // column tiles per warp
+    const int     mt = warp & 3, nt = (warp >> 2) * NT;
     double       *B  = fronts + n.koff + (int64_t)c0 * n.ld + b0;
     const double *LU = luf + n.luoff + (int64_t)b0 * n.nEp + b0;
     const double *TI = tinv + n.tioff + (int64_t)(b0 / NDPanel) * 2 * NDPanel * NDPanel;
     const int     ldl = n.nEp;
-    for (int c = warp; c < NDSolveCols; c += 8)
+    for (int c = warp; c < CT; c += 8)
       for (int r = lane; r < nblk * NDPanel; r += 32)
         Bs[c * ldb + r] = (c < nc && r < nr) ? B[(int64_t)c * n.ld + r] : 0.;
 
@@ -1245,7 +1254,7 @@ namespace ddhdg
         if (p.d < 2)
           p = next(p);
       }
-    double acc[2][2] = {};
+    double acc[NT][2] = {};
     bool   fresh     = true; // the row's accumulators are not loaded yet
     for (int it = 0; t.d < 2; ++it)
       {
@@ -1259,7 +1268,7 @@ namespace ddhdg
         if (fresh && t.j != t.i)
           {
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < NT; ++j)
 #pragma unroll
               for (int e = 0; e < 2; ++e)
                 acc[j][e] = Bs[((nt + j) * 8 + 2 * q + e) * ldb + row];
@@ -1268,19 +1277,19 @@ namespace ddhdg
         if (t.j != t.i)
           {
             // all fragments of the block first: the loads overlap
-            double a[NDPanel / 4], b[NDPanel / 4][2];
+            double a[NDPanel / 4], b[NDPanel / 4][NT];
 #pragma unroll
             for (int ks = 0; ks < NDPanel / 4; ++ks)
               {
                 a[ks] = -A[(ks * 4 + q) * NDPanelLd + mt * 8 + g];
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
+                for (int j = 0; j < NT; ++j)
                   b[ks][j] = Bs[((nt + j) * 8 + g) * ldb + t.j * NDPanel + ks * 4 + q];
               }
 #pragma unroll
             for (int ks = 0; ks < NDPanel / 4; ++ks)
 #pragma unroll
-              for (int j = 0; j < 2; ++j)
+              for (int j = 0; j < NT; ++j)
                 dmma8x8x4(acc[j][0], acc[j][1], a[ks], b[ks][j]);
           }
         else
@@ -1288,24 +1297,24 @@ namespace ddhdg
             if (!fresh)
               {
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
+                for (int j = 0; j < NT; ++j)
 #pragma unroll
                   for (int e = 0; e < 2; ++e)
                     Bs[((nt + j) * 8 + 2 * q + e) * ldb + row] = acc[j][e];
                 __syncthreads();
               }
-            double o[2][2] = {};
+            double o[NT][2] = {};
 #pragma unroll
             for (int ks = 0; ks < NDPanel / 4; ++ks)
               {
                 const double a = A[(ks * 4 + q) * NDPanelLd + mt * 8 + g];
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
+                for (int j = 0; j < NT; ++j)
                   dmma8x8x4(o[j][0], o[j][1], a, Bs[((nt + j) * 8 + g) * ldb + t.i * NDPanel + ks * 4 + q]);
               }
             __syncthreads();
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < NT; ++j)
 #pragma unroll
               for (int e = 0; e < 2; ++e)
                 Bs[((nt + j) * 8 + 2 * q + e) * ldb + row] = o[j][e];
@@ -1496,6 +1505,70 @@ namespace ddhdg
                 Cm[(int64_t)c * n.ld + r] = acc[i][j][e];
             }
         }
+  }
+
+  // The triangular solves of a front without kept dofs (the root): one
+  // column, resident in shared memory of one CTA per front.  Per block of
+  // NDPanel rows the inverted diagonal block (a warp per row), then the other
+  // rows a thread each: a chain of 2 nE / NDPanel L2 round trips, where the
+  // column tiles above would pad one column to 32 and sweep it in several
+  // launches (2304 rows: 1.3 ms before).
+  constexpr int NDRootT = 512;
+
+  __global__ void __launch_bounds__(NDRootT, 1)
+  nd_root_solve_kernel(const NDNode *nodes, const double *luf, const double *tinv, double *fronts)
+  {
+    extern __shared__ __align__(16) double sm[]; // the column, padded to whole blocks
+    __shared__ double xb[NDPanel];
+    const NDNode &n    = nodes[blockIdx.x];
+    const int     nE   = n.nE, nblk = (nE + NDPanel - 1) / NDPanel, ldl = n.nEp;
+    const double *LU = luf + n.luoff, *TI = tinv + n.tioff;
+    double       *B  = fronts + n.koff;
+    const int     tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int r = tid; r < nblk * NDPanel; r += NDRootT)
+      sm[r] = r < nE ? B[r] : 0.;
+    __syncthreads();
+    for (int s = 0; s < 2 * nblk; ++s)
+      {
+        const bool    up = s >= nblk;
+        const int     i  = up ? 2 * nblk - 1 - s : s, r0 = i * NDPanel;
+        const double *inv = TI + ((int64_t)i * 2 + (up ? 1 : 0)) * NDPanel * NDPanel;
+        for (int row = warp; row < NDPanel; row += NDRootT / 32)
+          {
+            double v = inv[lane * NDPanel + row] * sm[r0 + lane];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+              v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0)
+              xb[row] = v;
+          }
+        __syncthreads();
+        if (tid < NDPanel)
+          sm[r0 + tid] = xb[tid];
+        const int f = up ? 0 : r0 + NDPanel, l = up ? r0 : nE, w = min(NDPanel, nE - r0);
+        for (int r = f + tid; r < l; r += NDRootT)
+          {
+            const double *col = LU + (int64_t)r0 * ldl + r;
+            double        a   = 0.;
+            if (w == NDPanel)
+              {
+                double f[NDPanel]; // all loads in flight
+#pragma unroll
+                for (int k = 0; k < NDPanel; ++k)
+                  f[k] = col[(int64_t)k * ldl];
+#pragma unroll
+                for (int k = 0; k < NDPanel; ++k)
+                  a += f[k] * xb[k];
+              }
+            else
+              for (int k = 0; k < w; ++k)
+                a += col[(int64_t)k * ldl] * xb[k];
+            sm[r] -= a;
+          }
+        __syncthreads();
+      }
+    for (int r = tid; r < nE; r += NDRootT)
+      B[r] = sm[r];
   }
 
   // ------------------------------------------------------ back substitution

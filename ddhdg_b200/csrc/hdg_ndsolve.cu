@@ -33,7 +33,7 @@ namespace ddhdg
 
     constexpr int    PanelRows  = NDPanelT * NDPanelC; // rows the panel kernel can hold
     constexpr size_t SmallSmem  = 200 * 1024;
-    constexpr int    SolveRows  = 576; // rows of B that stay in shared memory (32 columns, 185 KB with the stages)
+    constexpr int    RootRows   = 24576; // rows of a single right-hand side in shared memory (192 KB)
 
     Class
     class_of(int nE, int nK)
@@ -583,7 +583,8 @@ namespace ddhdg
                          (const void *)nd_small_kernel<12, true>,  (const void *)nd_small_kernel<20, true>,
                          (const void *)nd_small_kernel<28, true>,  (const void *)nd_small_kernel<36, true>,
                          (const void *)nd_gather_b_kernel,         (const void *)nd_update_kernel,
-                         (const void *)nd_solve_kernel,            (const void *)nd_gemm_kernel<true>,
+                         (const void *)nd_solve_kernel<32>,        (const void *)nd_solve_kernel<64>,
+                         (const void *)nd_root_solve_kernel,       (const void *)nd_gemm_kernel<true>,
                          (const void *)nd_gemm_kernel<false>,      (const void *)nd_backsolve_kernel};
     for (const void *f : fns)
       if (allow_full_dynamic_smem(f) != cudaSuccess)
@@ -807,31 +808,42 @@ namespace ddhdg
           nd_gather_b_kernel<<<dim3(ceil_div(b.maxK + 1, cb), nb), 256, (size_t)cb * b.maxE * sizeof(double), s>>>(
             nodes, D.maps, C, D.perm, cb, D.fronts);
         }
-        const int cols = ceil_div(b.maxK + 1, NDSolveCols);
-        if (b.maxE <= SolveRows)
-          nd_solve_kernel<<<dim3(cols, nb), 256, nd_solve_smem(b.maxE), s>>>(nodes, 0, b.maxE, 3, D.luf, D.tinv,
-                                                                            D.fronts);
+        if (b.maxK == 0 && b.maxE <= RootRows)
+          nd_root_solve_kernel<<<nb, NDRootT, (size_t)ceil_div(b.maxE, NDPanel) * NDPanel * sizeof(double), s>>>(
+            nodes, D.luf, D.tinv, D.fronts);
         else
           {
-            // blocked: block rows of at most SolveRows in shared memory, the
+            const bool wide  = (int64_t)ceil_div(b.maxK + 1, 64) * nb >= sm_count;
+            const int  CT    = wide ? 64 : 32, cols = ceil_div(b.maxK + 1, CT);
+            const auto sweep = [&](int b0, int bs, int dir) {
+              if (wide)
+                nd_solve_kernel<64><<<dim3(cols, nb), 256, nd_solve_smem(64, bs), s>>>(nodes, b0, bs, dir, D.luf,
+                                                                                      D.tinv, D.fronts);
+              else
+                nd_solve_kernel<32><<<dim3(cols, nb), 256, nd_solve_smem(32, bs), s>>>(nodes, b0, bs, dir, D.luf,
+                                                                                      D.tinv, D.fronts);
+            };
+            // blocked: block rows whose column tiles fit in shared memory, the
             // rest of the rows updated by products
-            const int nblk = ceil_div(b.maxE, SolveRows);
+            const int nblk = ceil_div(b.maxE, nd_solve_rows(CT));
             const int bs   = ceil_div(ceil_div(b.maxE, nblk), NDPanel) * NDPanel;
             const int tn   = ceil_div(b.maxK + 1, NDGN);
-            for (int dir = 1; dir <= 2; ++dir)
-              for (int i = 0; i < nblk; ++i)
-                {
-                  const int b0 = (dir == 1 ? i : nblk - 1 - i) * bs;
-                  nd_solve_kernel<<<dim3(cols, nb), 256, nd_solve_smem(bs), s>>>(nodes, b0, bs, dir, D.luf, D.tinv,
-                                                                                D.fronts);
-                  const int r0 = dir == 1 ? b0 + bs : 0, mr = dir == 1 ? b.maxE - r0 : b0;
-                  if (mr > 0)
-                    {
-                      const int tm = ceil_div(mr, NDGM);
-                      nd_gemm_kernel<false><<<dim3(tm * tn, nb), 128, nd_gemm_smem(), s>>>(
-                        nodes, D.maps, C, tm, r0, mr, b0, bs, D.ecols, D.luf, D.fronts);
-                    }
-                }
+            if (nblk == 1)
+              sweep(0, bs, 3);
+            else
+              for (int dir = 1; dir <= 2; ++dir)
+                for (int i = 0; i < nblk; ++i)
+                  {
+                    const int b0 = (dir == 1 ? i : nblk - 1 - i) * bs;
+                    sweep(b0, bs, dir);
+                    const int r0 = dir == 1 ? b0 + bs : 0, mr = dir == 1 ? b.maxE - r0 : b0;
+                    if (mr > 0)
+                      {
+                        const int tm = ceil_div(mr, NDGM);
+                        nd_gemm_kernel<false><<<dim3(tm * tn, nb), 128, nd_gemm_smem(), s>>>(
+                          nodes, D.maps, C, tm, r0, mr, b0, bs, D.ecols, D.luf, D.fronts);
+                      }
+                  }
           }
         if (b.maxK > 0)
           {
