@@ -181,6 +181,22 @@ namespace ddhdg
   {
     return __float_as_uint(fabsf(x));
   }
+  // 1 / x by Newton's iteration from the hardware's approximation (no branch:
+  // a pivot step is bound by its dependent instructions); 0 for x = 0
+  __device__ __forceinline__ double
+  pivot_reciprocal(double x)
+  {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(r, fma(-x, r, 1.), r);
+    r = fma(r, fma(-x, r, 1.), r);
+    return x != 0. ? r : 0.;
+  }
+  __device__ __forceinline__ float
+  pivot_reciprocal(float x)
+  {
+    return x != 0.f ? 1.f / x : 0.f;
+  }
   __device__ __forceinline__ void
   store_pair(double *p, double a, double b)
   {
@@ -859,15 +875,18 @@ namespace ddhdg
             const bool     me   = lane == bl;
             const JT pj = __shfl_sync(0xffffffffu, srow[0], bl);
             sing |= kmax < 32u || !isfinite(pj);
-            const JT hr = (pj != JT(0)) ? JT(1) / pj : JT(0);
-            const JT l  = srow[0] * hr;
+            const JT hr = pivot_reciprocal(pj);
+            // the pivot's own row becomes -row / pivot by the same update,
+            // row - (1 + 1 / pivot) row: |pivot| <= 1 (equilibrated rows), so
+            // 1 + 1 / pivot keeps the reciprocal's digits
+            const JT l = me ? -(JT(1) + hr) : -(srow[0] * hr);
 #pragma unroll
             for (int k = 1; k < NSMAX; ++k)
               {
                 const JT pk = __shfl_sync(0xffffffffu, srow[k], bl);
-                srow[k - 1]     = me ? -pk * hr : srow[k] - l * pk;
+                srow[k - 1] = srow[k] + l * pk;
               }
-            srow[NSMAX - 1] = me ? hr : l;
+            srow[NSMAX - 1] = me ? hr : -l;
             if (me)
               {
                 used  = true;
@@ -948,19 +967,11 @@ namespace ddhdg
 
         // ------------------------ keep Y for the reconstruction [col][row]
         {
-          double   *yc  = P.ycache + cell * (int64_t)Ns * P.ycols;
-          const int tot = Ns * P.ycols;
-          int       row = lane % Ns, col = lane / Ns;
-          for (int idx = lane; idx < tot; idx += 32)
-            {
-              yc[idx] = Y[row * ldr + col];
-              row += 32;
-              while (row >= Ns)
-                {
-                  row -= Ns;
-                  ++col;
-                }
-            }
+          double *yc = P.ycache + cell * (int64_t)Ns * P.ycols;
+          if (lane < Ns)
+#pragma unroll 4
+            for (int col = 0; col < P.ycols; ++col)
+              yc[col * Ns + lane] = Y[lane * ldr + col];
         }
         // combined residual column with the Dirichlet columns folded in
         for (int j = lane; j < Ns; j += 32)
