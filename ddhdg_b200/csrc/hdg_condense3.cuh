@@ -197,16 +197,6 @@ namespace ddhdg
   {
     return x != 0.f ? 1.f / x : 0.f;
   }
-  __device__ __forceinline__ void
-  store_pair(double *p, double a, double b)
-  {
-    *reinterpret_cast<double2 *>(p) = make_double2(a, b);
-  }
-  __device__ __forceinline__ void
-  store_pair(float *p, float a, float b)
-  {
-    *reinterpret_cast<float2 *>(p) = make_float2(a, b);
-  }
 
   // JT: the Jacobian type.  double: the FP64 kernel.  float: the mixed
   // kernel, where the linearised operators, S and its inverse, R / Y, T and
@@ -237,6 +227,13 @@ namespace ddhdg
     constexpr int NSMAX = 3 * nb;
     constexpr bool RW   = DIM == 3 && sizeof(JT) == 8; // recompute rA / rS / rD (see ws3_layout)
     static_assert(NSMAX <= 32, "one lane per row of the scalar system");
+    // A row's fluxes depend on the potential and on its own component, the
+    // other densities couple through the recombination alone.  In 3D the
+    // channels of the vanishing couplings are left out: two full passes over
+    // the channels per row instead of three (31^3 degree 1: 3.90 -> 3.47 ms);
+    // the shorter passes of 2D lose more to the split than they save (256^2
+    // degree 2: 2.98 against 3.09 ms).
+    constexpr bool PZ = DIM == 3;
 
     const int  lane  = threadIdx.x & 31;
     const int  ncomp = P.ncomp;
@@ -288,8 +285,11 @@ namespace ddhdg
     const int  cpk    = (P.comps[0] & 3) | ((P.comps[1] & 3) << 2) | ((P.comps[2] & 3) << 4);
     const auto cmp_of = [cpk](int c) { return (cpk >> (2 * c)) & 3; };
     bool         nen = false, pen = false;
+    int          cV = -1; // the enabled component V
     for (int c = 0; c < ncomp; ++c)
       {
+        if (cmp_of(c) == 0)
+          cV = c;
         nen |= cmp_of(c) == 1;
         pen |= cmp_of(c) == 2;
       }
@@ -700,8 +700,21 @@ namespace ddhdg
               R[lane * ldr] = (JT)v;
             }
             // trace columns, one trial component at a time
-            for (int cj = 0; cj < ncomp; ++cj)
+            for (int cj = 0; PZ && cj < ncomp; ++cj)
+              if (cmp_of(cj) != 0 && cj != ci)
+#pragma unroll
+                for (int t = 0; t < Ft; ++t)
+                  {
+                    const int col                          = ((t / nf) * ncomp + cj) * nf + t % nf;
+                    R[lane * ldr + 1 + col] = JT(0);
+                    if (two)
+                      R[lane * ldr + 1 + Nt + col] = JT(0);
+                  }
+            for (int pass = PZ && cV < 0 ? 1 : 0; pass < (PZ ? 2 : ncomp); ++pass)
               {
+                const int cj = PZ ? (pass == 0 ? cV : ci) : pass;
+                if (PZ && pass == 1 && bi == 0)
+                  continue;
                 const int     pr  = bi * 3 + cmp_of(cj);
                 const JT     *kap = ka + pr * nqc;
                 const JT     *rhp = rh + pr * Fq;
@@ -782,8 +795,11 @@ namespace ddhdg
         if (act)
           {
 #pragma unroll 1
-            for (int cj = 0; cj < ncomp; ++cj)
+            for (int pass = PZ && cV < 0 ? 1 : 0; pass < (PZ ? 2 : ncomp); ++pass)
               {
+                const int cj = PZ ? (pass == 0 ? cV : ci) : pass;
+                if (PZ && pass == 1 && bi == 0)
+                  continue;
                 const int     pr  = bi * 3 + cmp_of(cj);
                 const JT     *alp = al + pr * nqc;
                 const JT     *kap = ka + pr * nqc;
@@ -825,6 +841,30 @@ namespace ddhdg
                       acc[e] += g_ * C.phi_f[fq * nb + e] + r_ * C.RTr[fq * nb + e];
                   }
                 // block cj of the row (selects: no dynamic register index)
+#pragma unroll
+                for (int k = 0; k < NSMAX; ++k)
+                  if (k / nb == cj)
+                    srow[k] = (JT)acc[k % nb];
+              }
+            // the plain coupling to the other densities
+#pragma unroll 1
+            for (int cj = 0; PZ && cj < ncomp; ++cj)
+              {
+                if (cmp_of(cj) == 0 || cj == ci)
+                  continue;
+                const JT *alp = al + (bi * 3 + cmp_of(cj)) * nqc;
+                double    acc[nb];
+#pragma unroll
+                for (int e = 0; e < nb; ++e)
+                  acc[e] = 0.;
+#pragma unroll
+                for (int q = 0; q < nqc; ++q)
+                  {
+                    const double lt = (double)alp[q] * TLc[q * nb + a];
+#pragma unroll
+                    for (int e = 0; e < nb; ++e)
+                      acc[e] += lt * C.phi_c[q * nb + e];
+                  }
 #pragma unroll
                 for (int k = 0; k < NSMAX; ++k)
                   if (k / nb == cj)
@@ -877,8 +917,8 @@ namespace ddhdg
             sing |= kmax < 32u || !isfinite(pj);
             const JT hr = pivot_reciprocal(pj);
             // the pivot's own row becomes -row / pivot by the same update,
-            // row - (1 + 1 / pivot) row: |pivot| <= 1 (equilibrated rows), so
-            // 1 + 1 / pivot keeps the reciprocal's digits
+            // row - (1 + 1 / pivot) row: the rows are equilibrated, |pivot| is
+            // about 1 or less, and 1 + 1 / pivot keeps the reciprocal's digits
             const JT l = me ? -(JT(1) + hr) : -(srow[0] * hr);
 #pragma unroll
             for (int k = 1; k < NSMAX; ++k)
