@@ -67,8 +67,7 @@ class CondenseBatch:
         solvers' trace-solve graphs stay valid)."""
         import torch
 
-        s = g.sizes(thermo)
-        nc, Nt, dev = g.ncells, s.Nt, g.device
+        nc, Nt, dev = g.ncells, g._trace_size(thermo), g.device
         return {"tt": torch.empty((nc, Nt, Nt), dtype=torch.float64, device=dev),
                 "rhs": torch.empty((nc, Nt), dtype=torch.float64, device=dev),
                 "dflag": torch.empty((nc, Nt), dtype=torch.int32, device=dev),

@@ -110,7 +110,7 @@ namespace
     int64_t               nnz      = 0;
     DevBuf<int32_t>       rowptr, colind;
     DevBuf<uint8_t>       slots; // [ncells][F][F]
-    DevBuf<double>        ycache, tt, rhs, dval, csr, grhs, x, dtrace, dcell;
+    DevBuf<double>        ycache, tt, rhs, dval, x, dtrace, dcell;
     DevBuf<double>        rscratch; // per-CTA R blocks of the condense kernel, if needed
     std::unique_ptr<NDSolver> nd;   // nested-dissection trace solver (built on first use)
     DevBuf<int32_t>       dflag;
@@ -118,7 +118,7 @@ namespace
     DevBuf<int32_t>       d_perm, d_iperm, prow, pcol;
     DevBuf<int32_t>       pmap; // permuted position of each CSR entry
     DevBuf<double>        pval, pb, px;
-    bool                  built = false;
+    bool                  built = false, csr_built = false;
   };
 } // namespace
 
@@ -309,14 +309,43 @@ namespace
     rec(all);
   }
 
-  // Global trace sparsity (DoFTools::make_sparsity_pattern on the
-  // restricted trace dofs, src/np_solver.cpp:643-651) and the scatter slots.
+  // The sizes of a mode.  A face couples to the faces of its one or two
+  // cells, which share only it.
   int
   build_mode(ddhdg_ctx *c, int thermo)
   {
     Mode &m = c->mode[thermo];
     set_mode_comps(c, thermo);
     m.nd.reset();
+    const int64_t nd  = (int64_t)m.ncomp * c->nf;
+    int64_t       nnz = 0;
+    for (int64_t f = 0; f < c->nfaces; ++f)
+      nnz += (c->face_cells[f * 2] >= 0 && c->face_cells[f * 2 + 1] >= 0 ? 2 * c->F - 1 : c->F) * nd * nd;
+    if (nnz > INT32_MAX)
+      return fail(DDHDG_BAD_ARG, "global trace matrix too large for 32-bit CSR");
+    m.nnz       = nnz;
+    m.csr_built = false;
+    m.built     = true;
+    return DDHDG_OK;
+  }
+
+  // Global trace sparsity (DoFTools::make_sparsity_pattern on the
+  // restricted trace dofs, src/np_solver.cpp:643-651) and the scatter slots,
+  // built for the callers of the assembled matrix only: the condensation, the
+  // trace solve from the condensed blocks and the Newton loop need none of it
+  // (256 x 256 cells of degree 2: most of the two seconds of a first pass).
+  int
+  ensure_csr(ddhdg_ctx *c, int thermo)
+  {
+    Mode &m = c->mode[thermo];
+    if (!m.built)
+      {
+        const int rb = build_mode(c, thermo);
+        if (rb)
+          return rb;
+      }
+    if (m.csr_built)
+      return DDHDG_OK;
     const int     F = c->F, nf = c->nf, nc = m.ncomp;
     const int64_t nfaces = c->nfaces;
     // neighbour faces of every face
@@ -345,8 +374,6 @@ namespace
           nnz += (int64_t)nbr[f].size() * nc * nf;
         }
     rowptr[ndofs] = (int32_t)nnz;
-    if (nnz > INT32_MAX)
-      return fail(DDHDG_BAD_ARG, "global trace matrix too large for 32-bit CSR");
     std::vector<int32_t> colind(nnz);
     for (int64_t f = 0; f < nfaces; ++f)
       for (int r = 0; r < nc * nf; ++r)
@@ -375,7 +402,6 @@ namespace
       return r;
     if ((r = m.slots.upload(slots.data(), slots.size())))
       return r;
-    m.nnz = nnz;
     // nested-dissection permutation of the dofs for the sparse QR solve
     std::vector<int64_t> forder;
     nd_order(c, forder);
@@ -415,7 +441,7 @@ namespace
       return r;
     if ((r = m.pmap.upload(pmap.data(), pmap.size())))
       return r;
-    m.built = true;
+    m.csr_built = true;
     return DDHDG_OK;
   }
 
@@ -507,6 +533,38 @@ namespace
         case 3: return condense_kernels<3>(k, cf, rf, mixed);
         default: return false;
       }
+  }
+
+  // CTAs per SM of a kernel with its shared-memory limit raised, remembered
+  // per thread: the occupancy query costs more than a launch on the smallest
+  // devices
+  int
+  ctas_per_sm(const void *fn, int threads, size_t smem, int &per_sm)
+  {
+    struct Entry
+    {
+      int         dev;
+      const void *fn;
+      int         threads;
+      size_t      smem;
+      int         per_sm;
+    };
+    static thread_local std::vector<Entry> known;
+    int                                    dev = 0;
+    CK(cudaGetDevice(&dev));
+    for (const auto &e : known)
+      if (e.fn == fn && e.smem == smem && e.threads == threads && e.dev == dev)
+        {
+          per_sm = e.per_sm;
+          return DDHDG_OK;
+        }
+    CK(allow_full_dynamic_smem(fn));
+    per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
+    if (known.size() >= 64)
+      known.clear();
+    known.push_back(Entry{dev, fn, threads, smem, per_sm});
+    return DDHDG_OK;
   }
 
   // Warps (cells) per CTA of the register kernel: as many as its launch bound
@@ -1095,7 +1153,9 @@ ddhdg_get_sizes(const ddhdg_ctx *cc, int thermo, ddhdg_sizes *s)
   ddhdg_ctx *c = const_cast<ddhdg_ctx *>(cc);
   thermo       = thermo ? 1 : 0;
   int r;
-  if (!c->mode[thermo].built && (r = build_mode(c, thermo)))
+  // also the sparsity: who asks for nnz goes on to the assembled matrix, and
+  // finds nothing left to allocate there (stream capture)
+  if ((r = ensure_csr(c, thermo)))
     return r;
   const Mode &m  = c->mode[thermo];
   s->ncells      = c->ncells;
@@ -1197,17 +1257,17 @@ condense_range(ddhdg_ctx *c, const double *cell_state, const double *trace_state
       if (r_global)
         {
           int per_sm = 0;
-          CK(allow_full_dynamic_smem(cf.fn));
-          CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cf.fn, threads, smem));
+          if ((r = ctas_per_sm(cf.fn, threads, smem, per_sm)))
+            return r;
           const int64_t g = std::min<int64_t>(units, (int64_t)std::max(per_sm, 1) * c->sm_count);
           if ((r = m.rscratch.alloc((size_t)g * c->nb * m.ncomp * m.ncol)))
             return r;
           P.rscratch = m.rscratch.p;
         }
     }
-  CK(allow_full_dynamic_smem(cf.fn));
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cf.fn, threads, smem));
+  if ((r = ctas_per_sm(cf.fn, threads, smem, per_sm)))
+    return r;
   if (per_sm < 1)
     return fail(DDHDG_BAD_ARG, "condense kernel does not fit on an SM");
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, (int64_t)per_sm * c->sm_count));
@@ -1343,9 +1403,9 @@ reconstruct_range(ddhdg_ctx *c, const double *cell_state, const double *trace_st
   const size_t smem =
     ((nPQ + 1) & ~(size_t)1) * sizeof(double) + (size_t)wpb * wsz * sizeof(double);
   P.wpb = wpb;
-  CK(allow_full_dynamic_smem(reinterpret_cast<const void *>(rf)));
-  int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rf, wpb * 32, smem));
+  int per_sm = 0, r;
+  if ((r = ctas_per_sm(reinterpret_cast<const void *>(rf), wpb * 32, smem, per_sm)))
+    return r;
   const int64_t blocks_needed = (c1 - c0 + wpb - 1) / wpb;
   const int     grid =
     (int)std::max<int64_t>(1, std::min<int64_t>(blocks_needed, (int64_t)std::max(per_sm, 1) * c->sm_count));
@@ -1391,10 +1451,16 @@ hostio_setup(ddhdg_ctx *c)
   return DDHDG_OK;
 }
 
+// first cell of a chunk: quarters of the cells, rounded to whole waves of the
+// register condensation (cells per SM at a time x SMs), since every chunk is a
+// launch of its own and ends with its own partly filled wave (160 x 160 cells
+// of degree 2: four chunks of 5.4 waves took 24 waves, in whole waves 22)
 static int64_t
 hostio_chunk_begin(const ddhdg_ctx *c, int k)
 {
-  return c->ncells * k / ddhdg_ctx::HostIO::NChunk;
+  const int64_t wave = 3 * c->nb <= 32 ? (int64_t)condense3_max_warps(c->nb, 8) * c->sm_count : 1;
+  const int64_t at   = c->ncells * k / ddhdg_ctx::HostIO::NChunk;
+  return k == ddhdg_ctx::HostIO::NChunk ? c->ncells : std::min(c->ncells, (at + wave / 2) / wave * wave);
 }
 
 int
@@ -1481,7 +1547,7 @@ ddhdg_get_csr(ddhdg_ctx *c, int thermo, const int32_t **row_ptr, const int32_t *
     return fail(DDHDG_BAD_ARG, "null argument");
   thermo = thermo ? 1 : 0;
   int r;
-  if (!c->mode[thermo].built && (r = build_mode(c, thermo)))
+  if ((r = ensure_csr(c, thermo)))
     return r;
   *row_ptr = c->mode[thermo].rowptr.p;
   *col_idx = c->mode[thermo].colind.p;
@@ -1498,7 +1564,7 @@ ddhdg_scatter(ddhdg_ctx *c, const double *tt, const double *rhs, const int32_t *
   thermo  = thermo ? 1 : 0;
   Mode &m = c->mode[thermo];
   int   r;
-  if (!m.built && (r = build_mode(c, thermo)))
+  if ((r = ensure_csr(c, thermo)))
     return r;
   cudaStream_t s = (cudaStream_t)stream;
   CK(cudaMemsetAsync(csr, 0, m.nnz * sizeof(double), s));
@@ -1524,6 +1590,11 @@ ddhdg_solve_trace(ddhdg_ctx *c, const double *csr, const double *grhs, double *x
   Mode &m = c->mode[thermo];
   if (!m.built)
     return fail(DDHDG_BAD_ARG, "sparsity not built");
+  {
+    const int rc = ensure_csr(c, thermo);
+    if (rc)
+      return rc;
+  }
   cudaStream_t s = (cudaStream_t)stream;
   if (!c->sp)
     {
@@ -1576,8 +1647,7 @@ ddhdg_newton(ddhdg_ctx *c, double *cell_state, double *trace_state, int thermo,
   cudaStream_t  s       = (cudaStream_t)stream;
   const int64_t ncell_d = c->ncells * 3 * (c->dim + 1) * c->nb;
   const int64_t ntr_d   = c->nfaces * 3 * c->nf;
-  if ((r = m.csr.alloc(m.nnz)) || (r = m.grhs.alloc(m.ndofs)) || (r = m.x.alloc(m.ndofs)) ||
-      (r = m.dtrace.alloc(ntr_d)) || (r = m.dcell.alloc(ncell_d)) ||
+  if ((r = m.x.alloc(m.ndofs)) || (r = m.dtrace.alloc(ntr_d)) || (r = m.dcell.alloc(ncell_d)) ||
       (r = c->norm_buf.alloc(4)))
     return r;
   cudaEvent_t ev[4];
@@ -1825,9 +1895,9 @@ ddhdg_assemble_condense_noalloc(ddhdg_ctx *c, const double *cell_state,
       threads = condense2_threads(c->nb);
       units   = c->ncells;
     }
-  CK(allow_full_dynamic_smem(cf.fn));
   int per_sm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cf.fn, threads, smem));
+  if ((r = ctas_per_sm(cf.fn, threads, smem, per_sm)))
+    return r;
   if (per_sm < 1)
     return fail(DDHDG_BAD_ARG, "condense kernel does not fit on an SM");
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, (int64_t)per_sm * c->sm_count));

@@ -220,6 +220,10 @@ class NPSolver:
         _lib.check(self.L.ddhdg_get_sizes(self._ctx, int(thermo), ctypes.byref(s)), "get_sizes")
         return s
 
+    def _trace_size(self, thermo):
+        """condensed trace dofs per cell (sizes().Nt), without a library call"""
+        return self.F * self.nf * (1 if thermo else sum(self.enabled))
+
     def _sp(self):
         return ctypes.c_void_p(self.stream.cuda_stream)
 
@@ -266,17 +270,17 @@ class NPSolver:
     # ---------------------------------------------- per-step primitives
     def assemble_condense(self, thermo=False):
         torch = _torch()
-        s = self.sizes(thermo)
-        nc, Nt = self.ncells, s.Nt
-        tt = torch.empty(nc * Nt * Nt, dtype=torch.float64, device=self.device)
-        rhs = torch.empty(nc * Nt, dtype=torch.float64, device=self.device)
-        dflag = torch.empty(nc * Nt, dtype=torch.int32, device=self.device)
-        dval = torch.empty(nc * Nt, dtype=torch.float64, device=self.device)
+        nc, Nt = self.ncells, self._trace_size(thermo)
+        f64 = torch.float64
+        tt = torch.empty((nc, Nt, Nt), dtype=f64, device=self.device)
+        rhs = torch.empty((nc, Nt), dtype=f64, device=self.device)
+        dflag = torch.empty((nc, Nt), dtype=torch.int32, device=self.device)
+        dval = torch.empty((nc, Nt), dtype=f64, device=self.device)
         _lib.check(self.L.ddhdg_assemble_condense(self._ctx, self.cell_state.data_ptr(),
                                                   self.trace_state.data_ptr(), int(thermo),
                                                   tt.data_ptr(), rhs.data_ptr(), dflag.data_ptr(),
                                                   dval.data_ptr(), self._sp()), "assemble_condense")
-        return tt.view(nc, Nt, Nt), rhs.view(nc, Nt), dflag.view(nc, Nt), dval.view(nc, Nt)
+        return tt, rhs, dflag, dval
 
     def reconstruct(self, update_trace, thermo=False):
         torch = _torch()
