@@ -524,13 +524,13 @@ namespace
   }
 
   bool
-  kernels_for(int dim, int k, CondenseKernel &cf, ReconstructFn &rf, bool mixed = false)
+  kernels_for(int dim, int k, CondenseKernel &cf, ReconstructFn &rf, bool mixed = false, bool wide = false)
   {
     switch (dim)
       {
-        case 1: return condense_kernels<1>(k, cf, rf, mixed);
-        case 2: return condense_kernels<2>(k, cf, rf, mixed);
-        case 3: return condense_kernels<3>(k, cf, rf, mixed);
+        case 1: return condense_kernels<1>(k, cf, rf, mixed, wide);
+        case 2: return condense_kernels<2>(k, cf, rf, mixed, wide);
+        case 3: return condense_kernels<3>(k, cf, rf, mixed, wide);
         default: return false;
       }
   }
@@ -571,11 +571,16 @@ namespace
   // and shared memory allow (mixed: two CTAs per SM), but no more than spread
   // the cells over every SM (a small device is bound by one cell's latency,
   // which grows with the warps sharing an SM).
+  bool
+  condense3_wide(const ddhdg_ctx *c, int64_t cells, bool mixed)
+  {
+    return condense3_has_wide(c->nb, mixed ? 4 : 8) && cells > (int64_t)Condense3Warps * c->sm_count;
+  }
   int
   condense3_wpb(const ddhdg_ctx *c, size_t per, int64_t cells, bool mixed)
   {
     // 227 KB per CTA, less the kernel's static arrays (face-flux table, pivots)
-    const int     wmax = condense3_max_warps(c->nb, mixed ? 4 : 8);
+    const int     wmax = Condense3Warps * (condense3_wide(c, cells, mixed) ? 2 : 1);
     const int64_t stat = (int64_t)c->F * c->nqf * c->F * c->nf * 8 + wmax * 3 * c->nb * 4 + 64;
     const int64_t most = std::min<int64_t>(wmax, (mixed ? 110 * 1024 : 227 * 1024 - stat) / (int64_t)per);
     const int64_t spread = std::max<int64_t>(1, (cells + c->sm_count - 1) / c->sm_count);
@@ -1216,7 +1221,7 @@ condense_range(ddhdg_ctx *c, const double *cell_state, const double *trace_state
   CondenseKernel cf;
   ReconstructFn rf;
   const bool mixed = c->desc.precision == 1;
-  if (!kernels_for(c->dim, c->k, cf, rf, mixed))
+  if (!kernels_for(c->dim, c->k, cf, rf, mixed, condense3_wide(c, c1 - c0, mixed)))
     return fail(DDHDG_BAD_ARG, "unsupported dim/degree");
   KParams P     = make_params(c, thermo);
   P.cell0       = c0;
@@ -1458,7 +1463,7 @@ hostio_setup(ddhdg_ctx *c)
 static int64_t
 hostio_chunk_begin(const ddhdg_ctx *c, int k)
 {
-  const int64_t wave = 3 * c->nb <= 32 ? (int64_t)condense3_max_warps(c->nb, 8) * c->sm_count : 1;
+  const int64_t wave = 3 * c->nb <= 32 ? (int64_t)Condense3Warps * c->sm_count : 1;
   const int64_t at   = c->ncells * k / ddhdg_ctx::HostIO::NChunk;
   return k == ddhdg_ctx::HostIO::NChunk ? c->ncells : std::min(c->ncells, (at + wave / 2) / wave * wave);
 }
@@ -1859,7 +1864,7 @@ ddhdg_assemble_condense_noalloc(ddhdg_ctx *c, const double *cell_state,
   // the same kernel as ddhdg_assemble_condense: the FP32-Jacobian variant on
   // a mixed-precision context
   const bool mixed = c->desc.precision == 1;
-  if (!kernels_for(c->dim, c->k, cf, rf, mixed))
+  if (!kernels_for(c->dim, c->k, cf, rf, mixed, condense3_wide(c, c->ncells, mixed)))
     return fail(DDHDG_BAD_ARG, "unsupported dim/degree");
   int     r;
   KParams P     = make_params(c, thermo);

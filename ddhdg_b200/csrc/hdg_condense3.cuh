@@ -25,14 +25,17 @@
 
 namespace ddhdg
 {
-  // warps (cells) per CTA at most, by the nodes of a cell and the bytes of
-  // the Jacobian type: FP64 eight with 255 registers (2D k = 2, 3D k = 1),
-  // sixteen with 128 where the bodies need no more; mixed eight, two CTAs per
-  // SM
-  __host__ __device__ constexpr int
-  condense3_max_warps(int nb, int jb)
+  // Warps (cells) per CTA at most.  Eight, with 255 registers in FP64 (mixed:
+  // 128, two CTAs per SM).  The wide form of the smaller FP64 bodies (at most
+  // four nodes: 1D, 2D k = 1) has sixteen with 128 registers, for devices
+  // that fill the SMs (2D k = 1, 256 x 256 cells: 1.16 -> 0.84 ms); below
+  // eight cells per SM it only adds latency (32 x 32 cells, with the
+  // reconstruction: 32.9 against 30.9 us).
+  constexpr int Condense3Warps = 8;
+  __host__ __device__ constexpr bool
+  condense3_has_wide(int nb, int jb)
   {
-    return jb == 8 && nb <= 4 ? 16 : 8;
+    return jb == 8 && nb <= 4;
   }
 
   // row stride of the staged S^-1 (>= its padded width, = 4 mod 16 doubles:
@@ -1218,12 +1221,12 @@ namespace ddhdg
       }
   }
 
-  template <int DIM, int K, typename JT = double>
-  __global__ void __launch_bounds__(condense3_max_warps(Dims<DIM, K>::nb, sizeof(JT)) * 32, sizeof(JT) == 8 ? 1 : 2)
+  template <int DIM, int K, typename JT = double, bool WIDE = false>
+  __global__ void __launch_bounds__(Condense3Warps * (WIDE ? 2 : 1) * 32, sizeof(JT) == 8 ? 1 : 2)
   condense3_kernel(const KParams P, const __grid_constant__ CTab<DIM, K> C)
   {
     extern __shared__ __align__(16) double smem[];
-    __shared__ int    piv3[condense3_max_warps(Dims<DIM, K>::nb, sizeof(JT))][3 * Dims<DIM, K>::nb];
+    __shared__ int    piv3[Condense3Warps * (WIDE ? 2 : 1)][3 * Dims<DIM, K>::nb];
     __shared__ double rqr_s[CTab<DIM, K>::Fq * CTab<DIM, K>::Ft];
     for (int i = threadIdx.x; i < CTab<DIM, K>::Fq * CTab<DIM, K>::Ft; i += blockDim.x)
       rqr_s[i] = P.tables[P.to.RQr + i];

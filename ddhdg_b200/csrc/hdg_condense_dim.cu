@@ -9,7 +9,7 @@ namespace ddhdg
 {
   namespace
   {
-    template <int D, int K, typename JT>
+    template <int D, int K, typename JT, bool WIDE>
     void
     launch_condense(const Tables &T, const KParams &P, int grid, int threads, size_t smem, cudaStream_t s)
     {
@@ -17,7 +17,7 @@ namespace ddhdg
         {
           CTab<D, K> C;
           fill_ctab(T, C);
-          condense3_kernel<D, K, JT><<<grid, threads, smem, s>>>(P, C);
+          condense3_kernel<D, K, JT, WIDE><<<grid, threads, smem, s>>>(P, C);
         }
       else
         condense2_kernel<D, K><<<grid, threads, smem, s>>>(P);
@@ -25,7 +25,7 @@ namespace ddhdg
 
     template <int D, int K>
     bool
-    pick(CondenseKernel &cf, ReconstructFn &rf, bool mixed)
+    pick(CondenseKernel &cf, ReconstructFn &rf, bool mixed, bool wide)
     {
       // register kernel when one lane can own one row of the scalar system,
       // CTA-per-cell shared-memory kernel otherwise
@@ -35,19 +35,25 @@ namespace ddhdg
           if (mixed)
             {
               cf.fn     = reinterpret_cast<const void *>(condense3_kernel<D, K, float>);
-              cf.launch = launch_condense<D, K, float>;
+              cf.launch = launch_condense<D, K, float, false>;
+            }
+          else if (condense3_has_wide(Dims<D, K>::nb, 8) && wide)
+            {
+              constexpr bool W = condense3_has_wide(Dims<D, K>::nb, 8);
+              cf.fn            = reinterpret_cast<const void *>(condense3_kernel<D, K, double, W>);
+              cf.launch        = launch_condense<D, K, double, W>;
             }
           else
             {
               cf.fn     = reinterpret_cast<const void *>(condense3_kernel<D, K, double>);
-              cf.launch = launch_condense<D, K, double>;
+              cf.launch = launch_condense<D, K, double, false>;
             }
           return true;
         }
       else
         {
           cf.fn     = reinterpret_cast<const void *>(condense2_kernel<D, K>);
-          cf.launch = launch_condense<D, K, double>;
+          cf.launch = launch_condense<D, K, double, false>;
           return !mixed;
         }
     }
@@ -55,15 +61,15 @@ namespace ddhdg
 
   template <>
   bool
-  condense_kernels<DDHDG_DIM>(int k, CondenseKernel &cf, ReconstructFn &rf, bool mixed)
+  condense_kernels<DDHDG_DIM>(int k, CondenseKernel &cf, ReconstructFn &rf, bool mixed, bool wide)
   {
     if (k == 1)
-      return pick<DDHDG_DIM, 1>(cf, rf, mixed);
+      return pick<DDHDG_DIM, 1>(cf, rf, mixed, wide);
     if (k == 2)
-      return pick<DDHDG_DIM, 2>(cf, rf, mixed);
+      return pick<DDHDG_DIM, 2>(cf, rf, mixed, wide);
 #if DDHDG_DIM < 3
     if (k == 3)
-      return pick<DDHDG_DIM, 3>(cf, rf, mixed);
+      return pick<DDHDG_DIM, 3>(cf, rf, mixed, wide);
 #endif
     return false;
   }

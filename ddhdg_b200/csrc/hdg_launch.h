@@ -23,9 +23,10 @@ namespace ddhdg
   using ReconstructFn = void (*)(KParams, const double *, double *);
 
   // mixed: the FP32-Jacobian variant of the register kernel; false when the
-  // degree has none (the caller rejects mixed precision there)
+  // degree has none (the caller rejects mixed precision there).  wide: its
+  // wide form, where there is one (condense3_has_wide).
   template <int D>
-  bool condense_kernels(int k, CondenseKernel &cf, ReconstructFn &rf, bool mixed);
+  bool condense_kernels(int k, CondenseKernel &cf, ReconstructFn &rf, bool mixed, bool wide);
 
   template <int D>
   struct BatchKernels
