@@ -77,9 +77,8 @@ def trace_solver_bytes(dim: int, m: int, k: int, ncomp: int) -> int:
     return int(out.value)
 
 
-# Device bytes of one request beyond its arrays and its trace solver (whose
-# library handles trace_solver_bytes counts): CUDA graphs, the context's and
-# the batch's streams and events
+# Device bytes of one request beyond its arrays and its trace solver: CUDA
+# graphs, the context's and the batch's streams and events
 REQUEST_OVERHEAD = 256 << 20
 
 
