@@ -29,6 +29,7 @@ from __future__ import annotations
 import math
 import threading
 import time
+import weakref
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -342,6 +343,7 @@ class DiodeServer(ThreadedDiodeServer):
         self.steps = 0  # group steps
         self.peak_batch = 0
         self._deferred = []
+        self._held = 0  # estimates of the finished requests whose memory is not back yet
 
     def _group_key(self, a):
         return (a.phase, a.req.dim, 1 if a.est > self.big_bytes else 0)
@@ -385,6 +387,9 @@ class DiodeServer(ThreadedDiodeServer):
                 return False
         return True
 
+    def _unhold(self, est):
+        self._held -= est
+
     def _release_deferred(self):
         import torch
 
@@ -401,6 +406,7 @@ class DiodeServer(ThreadedDiodeServer):
         committed = 0
         groups = {}  # group key -> {"ids", "batch", "members" of the step in flight or None}
         self._deferred = []
+        self._held = 0
         self._start_accounting()
         t0 = time.perf_counter()
         i = 0
@@ -410,9 +416,15 @@ class DiodeServer(ThreadedDiodeServer):
             while i < len(reqs) and reqs[i].arrival <= now and len(active) < self.max_inflight:
                 req = reqs[i]
                 est = memory_estimate(req.dim, req.m, req.k)
-                if not self.admissible(est, committed) and self._deferred:
-                    self._release_deferred()
-                if not self.admissible(est, committed):
+                # with no request in flight the live free figure is exact
+                if not self.admissible(est, committed + (self._held if active else 0)):
+                    if not active:  # no step is running: the idle batches hold finished requests too
+                        self._deferred += [gs["batch"] for gs in groups.values()]
+                        groups.clear()
+                    gs = None
+                    if self._deferred:
+                        self._release_deferred()
+                if not self.admissible(est, committed + (self._held if active else 0)):
                     if not active:
                         errors.append((req.rid, "does not fit in device memory"))
                         i += 1
@@ -452,6 +464,7 @@ class DiodeServer(ThreadedDiodeServer):
                     gs = groups[gk] = {"ids": ids, "members": None,
                                        "batch": CondenseBatch([a.solver for a in members], thermo=thermo,
                                                               buffers=bufs)}
+                    del bufs
                 gs["batch"].newton_step_begin([a.alpha for a in members])
                 gs["members"] = members
                 self.steps += 1
@@ -487,10 +500,15 @@ class DiodeServer(ThreadedDiodeServer):
                 active.remove(a)
                 committed -= a.est
                 g = a.solver
+                # until the solver is gone its memory is not free, and the
+                # requests in flight may not have allocated all of theirs
+                self._held += a.est
+                weakref.finalize(g, self._unhold, a.est)
                 finish = time.perf_counter() - t0
                 state = (g.get_cell_state().copy(), g.get_trace_state().copy()) if self.keep_states else None
                 results[a.req.rid] = Result(a.req.rid, a.req.arrival, a.start, finish, a.total_it, conv,
                                             g.ncells, state)
+                del g
 
                 def drop(a=a):
                     a.solver = None

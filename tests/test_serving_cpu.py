@@ -127,3 +127,74 @@ def test_groups_step_independently_with_fake_batches(monkeypatch):
         assert set(ids) <= big or not (set(ids) & big)
     assert sorted(released) == [0, 1, 3]
     assert server.peak_inflight == 4
+
+
+class _FakeSolver:
+    """Takes half of its estimate at once and the rest at its step `grow`."""
+
+    used = 0
+    peak = 0
+    ncells = 1
+
+    def __init__(self, est, steps, grow):
+        self.have, self.left, self.grow = 0, steps, grow
+        self.take(est // 2)
+
+    def take(self, n):
+        self.have += n
+        _FakeSolver.used += n
+        _FakeSolver.peak = max(_FakeSolver.peak, _FakeSolver.used)
+
+    def step(self):
+        self.left -= 1
+        self.grow -= 1
+        if self.grow == 0:
+            self.take(self.have)
+
+    def __del__(self):
+        _FakeSolver.used -= self.have
+
+
+class _FakeBatch:
+    def __init__(self, solvers, thermo=False, buffers=None):
+        self.solvers = list(solvers)
+
+    @staticmethod
+    def buffers_for(g, thermo=False):
+        return {}
+
+    def newton_step_begin(self, alphas):
+        for g in self.solvers:
+            g.step()
+
+    def newton_step_end(self, wait=True):
+        return [(0.0 if g.left <= 0 else 1.0, 0.0, 1.0, 1.0) for g in self.solvers], [0] * len(self.solvers)
+
+    def close(self):
+        pass
+
+
+def test_finished_requests_count_until_their_memory_is_back(monkeypatch):
+    """The solver of a finished request lives until its batch is replaced
+    and the deferred memory goes back; the requests in flight may take the
+    rest of their estimates before that, so an arrival is admitted only
+    beside all of them."""
+
+    class Server(serving.DiodeServer):
+        def _start_request(self, a):
+            steps, grow = {0: (12, 6), 1: (2, 1), 2: (8, 2)}[a.req.rid]
+            a.solver = _FakeSolver(a.est, steps, grow)
+            a.eq_tol, a.alpha = (1e-3, 1e-3, 50), 1.0
+
+        def _finish_phase(self, a):
+            return True
+
+    monkeypatch.setattr(serving, "memory_estimate", lambda dim, m, k: 4 * GB)
+    monkeypatch.setattr("ddhdg_b200.batch.CondenseBatch", _FakeBatch)
+    server = Server(hbm_reserve=0, mem_info=lambda: (10 * GB - _FakeSolver.used, 10 * GB))
+    reqs = [serving.Request(i, 2, 8, 1, 0.0, 0.0) for i in range(3)]
+    res = server.run(reqs)
+    assert [r.rid for r in res] == [0, 1, 2] and all(r.converged for r in res)
+    assert server.peak_inflight == 2
+    assert _FakeSolver.peak <= 8 * GB
+    assert _FakeSolver.used == 0
