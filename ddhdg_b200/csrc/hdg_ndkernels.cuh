@@ -250,13 +250,14 @@ namespace ddhdg
     const int32_t *map = maps + n.map;
     constexpr int  KM  = (1 << NDKidBit) - 1;
     // row jr, column offset jc of child s; raw cells carry the row scaling,
-    // their Dirichlet rows are identity rows (scale 0, the diagonal apart)
+    // their Dirichlet rows are identity rows, marked by the scale -1 (a scale
+    // is never negative; it is 0 for a row that holds an infinity)
     const auto place = [&](int s, int j, const double *&rp, double &rs, int &co) {
       const int64_t cell = LEAF ? n.cell : (s ? n.ccell[1] : n.ccell[0]);
       if (cell >= 0)
         {
           rp = C.tt + (cell * C.Nt + j) * (int64_t)C.Nt;
-          rs = C.dflag[cell * C.Nt + j] ? 0. : nd_cell_scale(C, cell, j);
+          rs = C.dflag[cell * C.Nt + j] ? -1. : nd_cell_scale(C, cell, j);
           co = j;
         }
       else
@@ -281,7 +282,7 @@ namespace ddhdg
     // value of an entry from what its place holds: row scale, column offsets
     // of the row's own position and of the entry
     const auto entry = [&](double x, double rs, int own, int co) -> double {
-      if (cells && rs == 0.)
+      if (cells && rs < 0.)
         return own == co ? 1. : 0.;
       return rs * x;
     };
@@ -290,10 +291,10 @@ namespace ddhdg
     const auto rhs_at = [&](int s, const double *rp, double rs, int own) -> const double * {
       const int64_t cell = LEAF ? n.cell : (s ? n.ccell[1] : n.ccell[0]);
       if (cell >= 0)
-        return (rs == 0. ? C.dval : C.rhs) + cell * C.Nt + own;
+        return (rs < 0. ? C.dval : C.rhs) + cell * C.Nt + own;
       return rp + (int64_t)(s ? n.cnK[1] : n.cnK[0]) * (s ? n.cld[1] : n.cld[0]);
     };
-    const auto rhs_scale = [&](double rs) { return cells && rs == 0. ? 1. : rs; };
+    const auto rhs_scale = [&](double rs) { return cells && rs < 0. ? 1. : rs; };
     for (int idx = tid; idx < NEM * NEM; idx += T)
       {
         const int i = idx % NEM, c = idx / NEM;
