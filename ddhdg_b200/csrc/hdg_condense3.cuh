@@ -22,6 +22,7 @@
 
 #include "hdg_condense.cuh"
 #include "hdg_mma.cuh"
+#include "hdg_reciprocal.cuh"
 
 namespace ddhdg
 {
@@ -183,22 +184,6 @@ namespace ddhdg
   pivot_key_bits(float x)
   {
     return __float_as_uint(fabsf(x));
-  }
-  // 1 / x by Newton's iteration from the hardware's approximation (no branch:
-  // a pivot step is bound by its dependent instructions); 0 for x = 0
-  __device__ __forceinline__ double
-  pivot_reciprocal(double x)
-  {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    r = fma(r, fma(-x, r, 1.), r);
-    r = fma(r, fma(-x, r, 1.), r);
-    return x != 0. ? r : 0.;
-  }
-  __device__ __forceinline__ float
-  pivot_reciprocal(float x)
-  {
-    return x != 0.f ? 1.f / x : 0.f;
   }
 
   // JT: the Jacobian type.  double: the FP64 kernel.  float: the mixed
@@ -916,13 +901,18 @@ namespace ddhdg
             const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
             const int      bl   = 31 - (int)(kmax & 31u);
             const bool     me   = lane == bl;
-            const JT pj = __shfl_sync(0xffffffffu, srow[0], bl);
-            sing |= kmax < 32u || !isfinite(pj);
-            const JT hr = pivot_reciprocal(pj);
+            // the pivot column times SC: a pivot of the equilibrated rows
+            // that is subnormal is normal then, with the reciprocal hs / SC
+            constexpr JT SC = sizeof(JT) == 8 ? JT(ReciprocalScale) : JT(1);
+            const JT     xs = srow[0] * SC;
+            const JT     hs = reciprocal_scaled(__shfl_sync(0xffffffffu, xs, bl));
+            const JT     hr = hs * SC;
+            // no pivot, or one without a finite reciprocal
+            sing |= kmax < 32u || !isfinite(hr);
             // the pivot's own row becomes -row / pivot by the same update,
             // row - (1 + 1 / pivot) row: the rows are equilibrated, |pivot| is
             // about 1 or less, and 1 + 1 / pivot keeps the reciprocal's digits
-            const JT l = me ? -(JT(1) + hr) : -(srow[0] * hr);
+            const JT l = me ? -(JT(1) + hr) : -(xs * hs);
 #pragma unroll
             for (int k = 1; k < NSMAX; ++k)
               {

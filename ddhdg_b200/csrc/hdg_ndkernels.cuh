@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "hdg_mma.cuh"
+#include "hdg_reciprocal.cuh"
 
 namespace ddhdg
 {
@@ -176,18 +177,6 @@ namespace ddhdg
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
   }
 
-  // 1 / x by Newton's iteration from the hardware's approximation: no branch,
-  // so that it overlaps the pivot search; 0 for x = 0
-  __device__ __forceinline__ double
-  nd_reciprocal(double x)
-  {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    r = fma(r, fma(-x, r, 1.), r);
-    r = fma(r, fma(-x, r, 1.), r);
-    return x != 0. ? r : 0.;
-  }
-
   // ------------------------------------------------------------ small fronts
   // nE <= NEM <= 36: the whole elimination of a front in one CTA.
   // - F_EE goes into the registers of one warp (two for NEM > 32), a row per
@@ -324,7 +313,7 @@ namespace ddhdg
             const int      buf  = j & 1;
             const double   x0   = v[0];
             const unsigned key  = used ? 0u : nd_pivot_key(x0);
-            const double   hx   = nd_reciprocal(x0); // overlaps the reduction
+            const double   hx   = reciprocal_normal(x0); // overlaps the reduction
             const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
             const int      src  = __ffs(__ballot_sync(0xffffffffu, key == kmax)) - 1;
             if (lane == src)
@@ -334,7 +323,7 @@ namespace ddhdg
 #pragma unroll
                 for (int k = 0; k < NEM; k += 2)
                   dst[k / 2] = make_double2(k < NEM - j ? v[k] : 0., k + 1 < NEM - j ? v[k + 1] : 0.);
-                phr_s[buf][warp]  = hx;
+                phr_s[buf][warp]  = reciprocal(x0, hx);
                 pkey_s[buf][warp] = kmax;
                 pid_s[buf][warp]  = tid;
               }
@@ -358,7 +347,7 @@ namespace ddhdg
                 pos     = j;
                 dinv[j] = hr;
                 perm[j] = tid;
-                bad |= hr == 0. || !isfinite(hr); // zero, subnormal or non-finite pivot
+                bad |= hr == 0. || isnan(hr); // zero or non-finite pivot
               }
           }
 #pragma unroll 1
@@ -685,7 +674,7 @@ namespace ddhdg
         const int      buf  = jj & 1;
         const double   x0   = v[jj];
         const unsigned key  = used ? 0u : nd_panel_key(x0, threadIdx.x);
-        const double   hx   = nd_reciprocal(x0);
+        const double   hx   = reciprocal_normal(x0);
         const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
         if (key == kmax && key != 0u)
           {
@@ -699,7 +688,7 @@ namespace ddhdg
 #pragma unroll
                 for (int k = b * NDPanelG; k < (b + 1) * NDPanelG; k += PK)
                   dst[k / PK] = make_double2(v[k], v[k + 1]);
-            S.whr[buf][warp] = hx;
+            S.whr[buf][warp] = reciprocal(x0, hx);
           }
         if (lane == 0)
           S.wkey[buf][warp] = kmax;
@@ -832,8 +821,8 @@ namespace ddhdg
       nd_cluster_sync(); // also: no CTA's shared memory is written after this
     else
       __syncthreads();
-    if (rank == 0 && tid < w && (S.rd[tid] == 0. || !isfinite(S.rd[tid])))
-      atomicExch(sing, 1); // a zero, subnormal or non-finite pivot
+    if (rank == 0 && tid < w && (S.rd[tid] == 0. || isnan(S.rd[tid])))
+      atomicExch(sing, 1); // a zero or non-finite pivot
     if (mypos >= 0)
       perm[n.poff + k0 + mypos] = row;
     else if (has)
