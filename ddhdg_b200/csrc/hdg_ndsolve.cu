@@ -34,6 +34,7 @@ namespace ddhdg
     constexpr int    PanelRows  = NDPanelT * NDPanelC; // rows the panel kernel can hold
     constexpr size_t SmallSmem  = 200 * 1024;
     constexpr int    RootRows   = 24576; // rows of a single right-hand side in shared memory (192 KB)
+    constexpr int    BatchNodes = 65535; // fronts per launch of the panel kernels (grid y)
 
     Class
     class_of(int nE, int nK)
@@ -261,7 +262,8 @@ namespace ddhdg
       for (int id : ids)
         {
           HostNode &h = tree[id];
-          if (batches.empty() || h.height != last_h || batches.back().cls != cls[id])
+          if (batches.empty() || h.height != last_h || batches.back().cls != cls[id] ||
+              (cls[id] >= Panels && batches.back().count == BatchNodes))
             {
               Batch b;
               b.cls   = cls[id];
