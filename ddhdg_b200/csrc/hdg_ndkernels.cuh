@@ -1083,7 +1083,8 @@ namespace ddhdg
       atomicExch(sing, 1);
     for (int j = 0; j < node->nE; ++j)
       {
-        const int k = ipiv[j] - 1, x = pm[j];
+        // within the front, whatever the library makes of NaN entries
+        const int k = max(j, min(ipiv[j] - 1, node->nE - 1)), x = pm[j];
         pm[j]       = pm[k];
         pm[k]       = x;
       }

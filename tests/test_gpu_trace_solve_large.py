@@ -49,9 +49,15 @@ def _backward_error(torch, g, tt, rhs, fl, dv, x):
     return float((res / top).abs().max() / scale)
 
 
-# a rod whose 65 600 cells each eliminate four faces, 48 dofs: more fronts of
-# the panel kernels at one height than a launch has room for in its y dimension
-@pytest.mark.parametrize("n,k", [((65600, 1, 1), 1)])
+# - a rod whose 65 600 cells each eliminate four faces, 48 dofs: more fronts of
+#   the panel kernels at one height than a launch has room for in its y
+#   dimension
+# - 11^3: fronts of 432 and 792 eliminated dofs above the 288 and 576 rows that
+#   a column tile of the triangular solves holds (blocks of rows, products
+#   between them), beside kept dofs
+# - 40 x 19 x 19: fronts of 4332 eliminated dofs, the root and its two children
+#   (4332 kept dofs each), whose LU is the library's
+@pytest.mark.parametrize("n,k", [((65600, 1, 1), 1), ((11, 11, 11), 1), ((40, 19, 19), 1)])
 def test_solution_satisfies_the_cells_equations(n, k):
     torch, g = _setup(n, k)
     tt, rhs, fl, dv = g.assemble_condense()
