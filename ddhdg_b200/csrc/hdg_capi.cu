@@ -162,6 +162,7 @@ struct ddhdg_ctx
     cudaEvent_t          ev_cell_free = nullptr, ev_dtrace_free = nullptr;
     cudaEvent_t          ev_chunk[NChunk] = {}, ev_rec[NChunk] = {};
     bool                 ready = false, have_state = false;
+    int64_t              wave = 1; // cells of a condensation launch on the SMs at a time
     ~HostIO()
     {
       for (cudaEvent_t e : {ev_trace, ev_out, ev_cell_free, ev_dtrace_free})
@@ -1205,6 +1206,51 @@ ddhdg_set_enabled(ddhdg_ctx *c, int V, int n, int p)
   return DDHDG_OK;
 }
 
+// the condense launch of a number of cells
+struct CondenseShape
+{
+  CondenseKernel kernel;
+  int            wpb     = 1; // cells per CTA
+  int            threads = 0, per_sm = 0, grid = 0;
+  size_t         smem     = 0;
+  bool           r_global = false; // R in KParams::rscratch, a slice per CTA
+};
+
+static int
+condense_shape(const ddhdg_ctx *c, const Mode &m, int64_t cells, CondenseShape &L)
+{
+  ReconstructFn rf;
+  const bool    mixed = c->desc.precision == 1;
+  int           r;
+  if (!kernels_for(c->dim, c->k, L.kernel, rf, mixed, condense3_wide(c, cells, mixed)))
+    return fail(DDHDG_BAD_ARG, "unsupported dim/degree");
+  if (3 * c->nb <= 32)
+    {
+      // as many cells per CTA as shared memory allows
+      // mixed: two CTAs per SM (the FP32 kernel is built for 128 registers)
+      const Ws3Off w   = ws3_layout(c->dim, c->nb, c->nf, m.ncomp, m.ncol, mixed ? 4 : 8);
+      const size_t per = (size_t)w.total * sizeof(double);
+      L.wpb            = condense3_wpb(c, per, cells, mixed);
+      if (L.wpb < 1)
+        return fail(DDHDG_BAD_ARG, "the per-cell workspace does not fit in shared memory");
+      L.threads = L.wpb * 32;
+      L.smem    = (size_t)L.wpb * per;
+    }
+  else
+    {
+      if ((r = launch_shape(c, m, L.r_global, L.smem)))
+        return r;
+      L.threads = condense2_threads(c->nb);
+    }
+  if ((r = ctas_per_sm(L.kernel.fn, L.threads, L.smem, L.per_sm)))
+    return r;
+  if (L.per_sm < 1)
+    return fail(DDHDG_BAD_ARG, "condense kernel does not fit on an SM");
+  const int64_t units = (cells + L.wpb - 1) / L.wpb;
+  L.grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, (int64_t)L.per_sm * c->sm_count));
+  return DDHDG_OK;
+}
+
 // the condense launch over the cells [c0, c1)
 static int
 condense_range(ddhdg_ctx *c, const double *cell_state, const double *trace_state, int thermo,
@@ -1218,11 +1264,9 @@ condense_range(ddhdg_ctx *c, const double *cell_state, const double *trace_state
   if ((r = ensure_buffers(c, thermo)))
     return r;
   Mode      &m = c->mode[thermo];
-  CondenseKernel cf;
-  ReconstructFn rf;
-  const bool mixed = c->desc.precision == 1;
-  if (!kernels_for(c->dim, c->k, cf, rf, mixed, condense3_wide(c, c1 - c0, mixed)))
-    return fail(DDHDG_BAD_ARG, "unsupported dim/degree");
+  CondenseShape L;
+  if ((r = condense_shape(c, m, c1 - c0, L)))
+    return r;
   KParams P     = make_params(c, thermo);
   P.cell0       = c0;
   P.ncells      = c1;
@@ -1233,50 +1277,14 @@ condense_range(ddhdg_ctx *c, const double *cell_state, const double *trace_state
   P.dflag       = dflag;
   P.dval        = dval;
   P.ycache      = m.ycache.p;
-  int    threads;
-  size_t smem;
-  int64_t units;
-  if (3 * c->nb <= 32)
+  P.wpb         = L.wpb;
+  if (L.r_global)
     {
-      // as many cells per CTA as shared memory allows
-      // mixed: two CTAs per SM (the FP32 kernel is built for 128 registers)
-      const Ws3Off w   = ws3_layout(c->dim, c->nb, c->nf, m.ncomp, m.ncol, mixed ? 4 : 8);
-      const size_t per = (size_t)w.total * sizeof(double);
-      int          wpb = condense3_wpb(c, per, c1 - c0, mixed);
-      if (wpb < 1)
-        return fail(DDHDG_BAD_ARG, "the per-cell workspace does not fit in shared memory");
-      P.wpb   = wpb;
-      P.stage = 0;
-      threads = wpb * 32;
-      smem    = (size_t)wpb * per;
-      units   = (c1 - c0 + wpb - 1) / wpb;
-    }
-  else
-    {
-      bool r_global;
-      if ((r = launch_shape(c, m, r_global, smem)))
+      if ((r = m.rscratch.alloc((size_t)L.grid * c->nb * m.ncomp * m.ncol)))
         return r;
-      P.wpb   = 1;
-      threads = condense2_threads(c->nb);
-      units   = c1 - c0;
-      if (r_global)
-        {
-          int per_sm = 0;
-          if ((r = ctas_per_sm(cf.fn, threads, smem, per_sm)))
-            return r;
-          const int64_t g = std::min<int64_t>(units, (int64_t)std::max(per_sm, 1) * c->sm_count);
-          if ((r = m.rscratch.alloc((size_t)g * c->nb * m.ncomp * m.ncol)))
-            return r;
-          P.rscratch = m.rscratch.p;
-        }
+      P.rscratch = m.rscratch.p;
     }
-  int per_sm = 0;
-  if ((r = ctas_per_sm(cf.fn, threads, smem, per_sm)))
-    return r;
-  if (per_sm < 1)
-    return fail(DDHDG_BAD_ARG, "condense kernel does not fit on an SM");
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, (int64_t)per_sm * c->sm_count));
-  cf.launch(c->Tu, P, grid, threads, smem, (cudaStream_t)stream);
+  L.kernel.launch(c->Tu, P, L.grid, L.threads, L.smem, (cudaStream_t)stream);
   CK(cudaGetLastError());
   return DDHDG_OK;
 }
@@ -1457,13 +1465,14 @@ hostio_setup(ddhdg_ctx *c)
 }
 
 // first cell of a chunk: quarters of the cells, rounded to whole waves of the
-// register condensation (cells per SM at a time x SMs), since every chunk is a
-// launch of its own and ends with its own partly filled wave (160 x 160 cells
-// of degree 2: four chunks of 5.4 waves took 24 waves, in whole waves 22)
+// condensation (the cells that a quarter's launch has on the SMs at a time),
+// since every chunk is a launch of its own and ends with its own partly filled
+// wave (160 x 160 cells of degree 2: four chunks of 5.4 waves took 24 waves,
+// in whole waves 22)
 static int64_t
 hostio_chunk_begin(const ddhdg_ctx *c, int k)
 {
-  const int64_t wave = 3 * c->nb <= 32 ? (int64_t)Condense3Warps * c->sm_count : 1;
+  const int64_t wave = c->hio.wave;
   const int64_t at   = c->ncells * k / ddhdg_ctx::HostIO::NChunk;
   return k == ddhdg_ctx::HostIO::NChunk ? c->ncells : std::min(c->ncells, (at + wave / 2) / wave * wave);
 }
@@ -1476,11 +1485,15 @@ ddhdg_assemble_condense_host(ddhdg_ctx *c, const double *cell_state_host,
   if (!c || !cell_state_host || !trace_state_host || !tt || !rhs || !dflag || !dval)
     return fail(DDHDG_BAD_ARG, "null argument");
   int r;
-  if ((r = hostio_setup(c)))
+  thermo = thermo ? 1 : 0;
+  CondenseShape L;
+  if ((r = hostio_setup(c)) || (r = ensure_buffers(c, thermo)) ||
+      (r = condense_shape(c, c->mode[thermo], std::max<int64_t>(1, c->ncells / ddhdg_ctx::HostIO::NChunk), L)))
     return r;
   auto        &h  = c->hio;
   cudaStream_t s  = (cudaStream_t)stream;
   const size_t pc = (size_t)3 * (c->dim + 1) * c->nb; // doubles per cell
+  h.wave          = (int64_t)L.wpb * L.per_sm * c->sm_count;
   // the device copies are rewritten once the kernels that read them (the
   // previous condensation or reconstruction) are done
   CK(cudaStreamWaitEvent(h.h2d, h.ev_cell_free, 0));
@@ -1859,59 +1872,26 @@ ddhdg_assemble_condense_noalloc(ddhdg_ctx *c, const double *cell_state,
   Mode &m = c->mode[thermo];
   if (!m.built)
     set_mode_comps(c, thermo); // host bookkeeping only; no trace sparsity needed here
-  CondenseKernel cf;
-  ReconstructFn rf;
-  // the same kernel as ddhdg_assemble_condense: the FP32-Jacobian variant on
-  // a mixed-precision context
-  const bool mixed = c->desc.precision == 1;
-  if (!kernels_for(c->dim, c->k, cf, rf, mixed, condense3_wide(c, c->ncells, mixed)))
-    return fail(DDHDG_BAD_ARG, "unsupported dim/degree");
-  int     r;
-  KParams P     = make_params(c, thermo);
-  P.cell_state  = cell_state;
-  P.trace_state = trace_state;
-  P.tt          = tt;
-  P.rhs         = rhs;
-  P.dflag       = dflag;
-  P.dval        = dval;
-  const int64_t Ns = (int64_t)m.ncomp * c->nb;
-  int           threads;
-  size_t        smem;
-  int64_t       units;
-  bool          r_global = false;
-  if (3 * c->nb <= 32)
-    {
-      const Ws3Off w   = ws3_layout(c->dim, c->nb, c->nf, m.ncomp, m.ncol, mixed ? 4 : 8);
-      const size_t per = (size_t)w.total * sizeof(double);
-      int          wpb = condense3_wpb(c, per, c->ncells, mixed);
-      if (wpb < 1)
-        return fail(DDHDG_BAD_ARG, "the per-cell workspace does not fit in shared memory");
-      P.wpb   = wpb;
-      P.stage = 0;
-      threads = wpb * 32;
-      smem    = (size_t)wpb * per;
-      units   = (c->ncells + wpb - 1) / wpb;
-    }
-  else
-    {
-      if ((r = launch_shape(c, m, r_global, smem)))
-        return r;
-      P.wpb   = 1;
-      threads = condense2_threads(c->nb);
-      units   = c->ncells;
-    }
-  int per_sm = 0;
-  if ((r = ctas_per_sm(cf.fn, threads, smem, per_sm)))
+  // the same launch as ddhdg_assemble_condense
+  CondenseShape L;
+  int           r;
+  if ((r = condense_shape(c, m, c->ncells, L)))
     return r;
-  if (per_sm < 1)
-    return fail(DDHDG_BAD_ARG, "condense kernel does not fit on an SM");
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, (int64_t)per_sm * c->sm_count));
+  KParams P        = make_params(c, thermo);
+  P.cell_state     = cell_state;
+  P.trace_state    = trace_state;
+  P.tt             = tt;
+  P.rhs            = rhs;
+  P.dflag          = dflag;
+  P.dval           = dval;
+  P.wpb            = L.wpb;
+  const int64_t Ns = (int64_t)m.ncomp * c->nb;
 
   // scratch: Y cache [ncells][Ns][ycols], then (256-byte aligned) one R block
   // [Ns][ncol] per CTA when R lives outside shared memory
   const size_t ycache_n = (size_t)c->ncells * Ns * m.ycols;
   const size_t r_off    = (ycache_n + 31) & ~(size_t)31;
-  const size_t need_n   = r_global ? r_off + (size_t)grid * Ns * m.ncol : ycache_n;
+  const size_t need_n   = L.r_global ? r_off + (size_t)L.grid * Ns * m.ncol : ycache_n;
   if (need_n * sizeof(double) > DDHDG_NOALLOC_SCRATCH_BYTES)
     return fail(DDHDG_BAD_ARG,
                 "this problem needs " + std::to_string(need_n * sizeof(double)) +
@@ -1922,11 +1902,11 @@ ddhdg_assemble_condense_noalloc(ddhdg_ctx *c, const double *cell_state,
   if ((r = noalloc_scratch(&scratch)))
     return r;
   P.ycache   = scratch;
-  P.rscratch = r_global ? scratch + r_off : nullptr;
+  P.rscratch = L.r_global ? scratch + r_off : nullptr;
 
   // the status word must start at zero (a singular local system sets it)
   CK(cudaMemsetAsync(c->status.p, 0, sizeof(int), (cudaStream_t)stream));
-  cf.launch(c->Tu, P, grid, threads, smem, (cudaStream_t)stream);
+  L.kernel.launch(c->Tu, P, L.grid, L.threads, L.smem, (cudaStream_t)stream);
   CK(cudaGetLastError());
   return DDHDG_OK;
 }
