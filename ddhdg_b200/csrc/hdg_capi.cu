@@ -1070,7 +1070,7 @@ ddhdg_ctx_create(const ddhdg_problem_desc *d, ddhdg_ctx **out)
     if ((r0 = c->d_face_local.upload(loc.data(), loc.size())))
       return r0;
   }
-  // stage the tables in one block
+  // the tables in one block
   {
     std::vector<double> blob;
     auto put = [&](const std::vector<double> &v) {
@@ -2509,7 +2509,6 @@ ddhdg_batch_create(const ddhdg_batch_item *items, int n, int thermo, ddhdg_batch
           b->smem_c = std::max(b->smem_c, ((size_t)batch_warps(c->dim) * w.total +
                                            (size_t)(c->F * c->nqf) * (c->F * c->nf)) * sizeof(double));
           J.P.wpb        = 1;
-          J.P.stage      = 0;
         }
       else
         {
@@ -2536,7 +2535,6 @@ ddhdg_batch_create(const ddhdg_batch_item *items, int n, int thermo, ddhdg_batch
           if (!found)
             return fail(DDHDG_BAD_ARG, "the per-cell workspace does not fit in shared memory");
           J.P.wpb   = 1;
-          J.P.stage = 0;
           b->smem_c = std::max(b->smem_c, smem);
           if (r_global)
             {

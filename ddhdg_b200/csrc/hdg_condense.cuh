@@ -8,7 +8,7 @@
 //     S y = R,   R = [residual | ct columns (| drift columns)].
 // Every block of S and R is a contraction over "channels" (cell quadrature
 // points, their gradient directions, face quadrature points) of per-cell
-// coefficients with constant tables staged in shared memory:
+// coefficients with constant tables:
 //     S_{b b'}[a][e] = sum_ch coef_{b b'}(ch) TL[ch][a] RT[ch][e].
 // The coupling coefficients per channel are (test component b, trial b'):
 //     alpha  value x value      (plain V-n/p coupling, Boltzmann term, dR/dn)
@@ -591,8 +591,8 @@ namespace ddhdg
   // The body of the CTA-per-cell condensation: the CTA (T threads, a
   // multiple of 32: condense2_threads in condense2_kernel, fewer in the batched
   // launch) works through the cells cell_begin, cell_begin + cell_step, ...
-  // < cell_end with the workspace at smem (tables first when P.stage) and,
-  // for R outside shared memory, the R slice `slot` of P.rscratch.
+  // < cell_end with the workspace at smem and, for R outside shared memory, the
+  // R slice `slot` of P.rscratch.
   template <int DIM, int K, int T = condense2_threads(Dims<DIM, K>::nb)>
   __device__ __forceinline__ void
   condense2_cells(const KParams &P, double *smem, int64_t slot, int64_t cell_begin,
@@ -621,15 +621,8 @@ namespace ddhdg
     const int ldS   = Ns + 1;
     const bool two  = ncol > 1 + Nt;
 
-    // ---- constant tables, staged once per CTA
-    const double *tb = P.tables;
-    if (P.stage)
-      {
-        for (int i = tid; i < P.to.total; i += T)
-          smem[i] = P.tables[i];
-        __syncthreads();
-        tb = smem;
-      }
+    // ---- constant tables, read through L1
+    const double *tb     = P.tables;
     const double *phi_c  = tb + P.to.phi_c;
     const double *w_f    = tb + P.to.w_f;
     const double *xi     = tb + P.to.xi;
@@ -648,7 +641,7 @@ namespace ddhdg
     const double *QW_f   = tb + P.to.QW_f;
 
     const Ws2Off wo = ws2_layout(DIM, nb, nf, ncomp, ncol, P.rscratch != nullptr);
-    double *ws = smem + (P.stage ? ((P.to.total + 1) & ~1) : 0);
+    double *ws = smem;
     double *coef = ws + wo.coef, *lam = ws + wo.lam, *c0 = ws + wo.c0, *W0 = ws + wo.W0,
            *qc = ws + wo.qc, *c0f = ws + wo.c0f, *W0n = ws + wo.W0n, *tr0 = ws + wo.tr0,
            *Wrc = ws + wo.Wrc, *Wrf = ws + wo.Wrf, *taus = ws + wo.tau, *bcs = ws + wo.bcs,

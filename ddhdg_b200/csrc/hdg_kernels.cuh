@@ -12,7 +12,7 @@ namespace ddhdg
   constexpr double Q_  = 1.602176634E-19;
   constexpr double EV_ = 1.602176565E-19;
 
-  // offsets (in doubles) of the tables inside the staged table block
+  // offsets (in doubles) of the tables inside the table block
   struct TabOff
   {
     int phi_c, grad_c, w_c, phi_f, w_f, xi, fminvw, PW_c, PW_f, QW_c, QW_f, P,
@@ -45,7 +45,6 @@ namespace ddhdg
     int ncol;  // columns of the scalar system: 1 + Nt (+ Nt)
     int ycols; // columns kept for the reconstruction: 1 + Nt
     int wpb;   // warps per block
-    int stage; // 1: copy the tables to shared memory, 0: read them from L1/L2
     // state
     const double *cell_state, *trace_state;
     // outputs
