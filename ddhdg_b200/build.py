@@ -1,6 +1,7 @@
 """Builds the CUDA library ``libddhdg_b200.so`` in-tree for sm_100a."""
 
 import os
+import signal
 import subprocess
 import sys
 import tempfile
@@ -43,10 +44,18 @@ def build(force=False, verbose=False):
             cmd = [nvcc()] + NVCC_FLAGS + extra + ["-c", "-o", objs[-1], os.path.join(CSRC, s)]
             if verbose:
                 print(" ".join(cmd), file=sys.stderr)
-            jobs.append((cmd, subprocess.Popen(cmd)))
-        for cmd, job in jobs:
-            if job.wait():
-                raise subprocess.CalledProcessError(job.returncode, cmd)
+            jobs.append((cmd, subprocess.Popen(cmd, start_new_session=True)))
+        try:
+            for cmd, job in jobs:
+                if job.wait():
+                    raise subprocess.CalledProcessError(job.returncode, cmd)
+        finally:
+            # after a failure: no compiler (nvcc and the programs it runs) may
+            # outlive the directory it writes to
+            for _, job in jobs:
+                if job.poll() is None:
+                    os.killpg(job.pid, signal.SIGTERM)
+                job.wait()
         cmd = [nvcc()] + NVCC_FLAGS + ["-shared", "-o", LIB] + objs + ["-lcusolver", "-lcusparse"]
         if verbose:
             print(" ".join(cmd), file=sys.stderr)
