@@ -31,8 +31,8 @@
 namespace ddhdg
 {
   // Threads per CTA (cell) by the nodes of a cell: two warps where four cells
-  // share an SM (2D k = 3), eight where one cell fills its shared memory
-  // (3D k = 2).
+  // share an SM (2D k = 3), eight where one cell has it alone (3D k = 2, whose
+  // registers fill it).
   __host__ __device__ constexpr int
   condense2_threads(int nb)
   {
