@@ -29,7 +29,7 @@ namespace ddhdg
   // Warps (cells) per CTA at most.  Eight, with 255 registers in FP64 (mixed:
   // 128, two CTAs per SM).  The wide form of the smaller FP64 bodies (at most
   // four nodes: 1D, 2D k = 1) has sixteen with 128 registers, for devices
-  // that fill the SMs (2D k = 1, 256 x 256 cells: 1.16 -> 0.84 ms); below
+  // that fill the SMs (2D k = 1, 256 x 256 cells: 1.16 -> 0.80 ms); below
   // eight cells per SM it only adds latency (32 x 32 cells, with the
   // reconstruction: 32.9 against 30.9 us).
   constexpr int Condense3Warps = 8;
